@@ -96,6 +96,21 @@ __device__ __forceinline__ uint32_t udiv(uint32_t n, UDiv d) {
 }
 #endif
 
+// Constants of the FP64 collision, formed once by the host with the IEEE
+// operations (and order) the reference uses, so that no thread spends FP64
+// instructions on them
+struct Consts64 {
+    double we, wodd;   // rates of the even and odd parts (BGK, regularized: both 1/tau)
+    double c2;         // 1 - we/2
+    double c3, c4, r9; // 1 - (we + wo)/2, (we - wo)/2, 1 - we
+};
+// a force: acceleration a, c1 a and 2 c2 a, and a bit for each component that
+// is not known to be zero
+struct Force64 {
+    double a[3], c1a[3], c2a[3];
+    unsigned mask;
+};
+
 struct StepArgs {
     void *f;              // populations, 19 * Np elements of the storage type
     int64_t Np;           // slot stride
@@ -109,6 +124,9 @@ struct StepArgs {
     float gf[3];          // g, w_e and w_o rounded to float once by the host:
     float w_ef, w_of;     // the float kernels read these (a per-thread double
                           // conversion runs on the narrow FP64 pipe)
+    Consts64 k64;         // FP64 collision constants
+    double c1;            // first-moment force factor: 1 - wo/2 (TRT), 1 - we/2
+    Force64 g64;          // uniform gravity with its factors
     int write_moments;
     // dense-node grid
     int bx, by, kblocks;  // block shape and k-blocks per row-block
@@ -144,6 +162,27 @@ struct StepArgs {
     void *sp_tee;         // if set: collision inputs (after Zou-He) of the
                           // boundary nodes, [19][M] in the storage type
 };
+
+// fills a.k64, a.c1 and a.g64 from the rates and gravity of `a`; compiled
+// without contraction, as the reference's host arithmetic
+inline void set_consts64(StepArgs &a, int scheme) {
+    Consts64 &k = a.k64;
+    k.we = a.w_e;
+    k.wodd = scheme == SCH_TRT ? a.w_o : a.w_e;
+    k.c2 = 1.0 - 0.5 * a.w_e;
+    k.c3 = 1.0 - 0.5 * (a.w_e + a.w_o);
+    k.c4 = 0.5 * (a.w_e - a.w_o);
+    k.r9 = 1.0 - a.w_e;
+    // the regularized update weighs the first-moment force by 1 - we/2 too
+    a.c1 = scheme == SCH_TRT ? 1.0 - 0.5 * a.w_o : k.c2;
+    a.g64.mask = 0;
+    for (int d = 0; d < 3; ++d) {
+        a.g64.a[d] = a.g[d];
+        a.g64.c1a[d] = a.c1 * a.g[d];
+        a.g64.c2a[d] = 2.0 * k.c2 * a.g[d];
+        if (a.g[d] != 0.0) a.g64.mask |= 1u << d;
+    }
+}
 
 // Blocks of the boundary-node path in a launch of the direct step kernel (or
 // the adjoint's reverse kernel), whose blocks have a.bx * a.by threads: 96

@@ -612,6 +612,7 @@ StepArgs make_args(const jlb_solver *s, int write_moments) {
     for (int d = 0; d < 3; ++d) a.gf[d] = (float)a.g[d];
     a.w_ef = (float)a.w_e;
     a.w_of = (float)a.w_o;
+    set_consts64(a, s->cfg.rlx_scheme);
     a.write_moments = write_moments;
     const int nzr = ((s->nz + 31) / 32) * 32;
     a.bx = nzr >= 128 ? 128 : nzr;

@@ -141,6 +141,31 @@ template <class C> __device__ __forceinline__ C arg_g(const StepArgs &a, int d) 
 template <class C> __device__ __forceinline__ C arg_we(const StepArgs &a) { return par<C>(a.w_e, a.w_ef); }
 template <class C> __device__ __forceinline__ C arg_wo(const StepArgs &a) { return par<C>(a.w_o, a.w_of); }
 
+// physics policies that take the host's FP64 constants (StepArgs::k64) and a
+// Force64 declare host_consts = true
+template <class PH, class = void> struct uses_host_consts {
+    static constexpr bool value = false;
+};
+template <class PH> struct uses_host_consts<PH, std::void_t<decltype(PH::host_consts)>> {
+    static constexpr bool value = PH::host_consts;
+};
+// the force of site n: the uniform one with the host's factors, or with the
+// acceleration field added (its factors are formed here, in the same order)
+template <bool ACCF> __device__ __forceinline__ Force64 site_force64(const StepArgs &a, int64_t n) {
+    Force64 F = a.g64;
+    if (ACCF) {
+        const double *acc = (const double *)a.acc;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            F.a[d] = a.g[d] + __ldg(acc + d * a.Np + n);
+            F.c1a[d] = a.c1 * F.a[d];
+            F.c2a[d] = 2.0 * a.k64.c2 * F.a[d];
+        }
+        F.mask = 7u;
+    }
+    return F;
+}
+
 // compile-time loop
 template <int I, int N> struct Unroll {
     template <class F> __device__ __forceinline__ static void run(F &&f) {
@@ -239,6 +264,8 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
         }
         rho = PH::collide_fd(fv, arg_g<C>(a, 0), arg_g<C>(a, 1), arg_g<C>(a, 2), fx, fy, fz, arg_we<C>(a),
                              arg_wo<C>(a), ux, uy, uz);
+    } else if constexpr (uses_host_consts<PH>::value) {
+        rho = PH::collide(fv, site_force64<ACCF>(a, n), a.k64, ux, uy, uz);
     } else {
         C ax, ay, az;
         if (ACCF) {
@@ -337,6 +364,8 @@ __device__ __forceinline__ void special_node(const StepArgs &a, int b) {
         }
         rho = PH::collide_fd(fv, arg_g<C>(a, 0), arg_g<C>(a, 1), arg_g<C>(a, 2), fx, fy, fz, arg_we<C>(a),
                              arg_wo<C>(a), ux, uy, uz);
+    } else if constexpr (uses_host_consts<PH>::value) {
+        rho = PH::collide(fv, site_force64<ACCF>(a, n), a.k64, ux, uy, uz);
     } else {
         C ax, ay, az;
         if (ACCF) {
