@@ -21,6 +21,8 @@
 #include <cmath>
 #include <cuda_runtime.h>
 
+#include "soft64.cuh"
+
 namespace jlb {
 
 constexpr int Q = 19;
@@ -103,6 +105,11 @@ struct Consts64 {
     double we, wodd;   // rates of the even and odd parts (BGK, regularized: both 1/tau)
     double c2;         // 1 - we/2
     double c3, c4, r9; // 1 - (we + wo)/2, (we - wo)/2, 1 - we
+    // the same for the integer product (soft64::mul), with the projection's
+    // 1/72 and 1/36; `nonzero` has a bit for each of c3, c4, r9 that is not 0
+    soft64::MulC mc3, mc4, mr9, m72, m36;
+    unsigned nonzero;
+    int soft; // 1: every constant is zero or well inside the normal range
 };
 // a force: acceleration a, c1 a and 2 c2 a, and a bit for each component that
 // is not known to be zero
@@ -173,6 +180,18 @@ inline void set_consts64(StepArgs &a, int scheme) {
     k.c3 = 1.0 - 0.5 * (a.w_e + a.w_o);
     k.c4 = 0.5 * (a.w_e - a.w_o);
     k.r9 = 1.0 - a.w_e;
+    k.m72 = soft64::make_mulc(1.0 / 72.0);
+    k.m36 = soft64::make_mulc(2.0 * (1.0 / 72.0));
+    k.mc3 = soft64::make_mulc(k.c3);
+    k.mc4 = soft64::make_mulc(k.c4);
+    k.mr9 = soft64::make_mulc(k.r9);
+    k.nonzero = 0;
+    k.soft = 1;
+    const double rel[3] = {k.c3, k.c4, k.r9};
+    for (int i = 0; i < 3; ++i) {
+        if (rel[i] != 0.0) k.nonzero |= 1u << i;
+        if (rel[i] != 0.0 && !(std::fabs(rel[i]) > 0x1p-200 && std::fabs(rel[i]) < 0x1p10)) k.soft = 0;
+    }
     // the regularized update weighs the first-moment force by 1 - we/2 too
     a.c1 = scheme == SCH_TRT ? 1.0 - 0.5 * a.w_o : k.c2;
     a.g64.mask = 0;

@@ -18,9 +18,13 @@ namespace jlb {
 //     from 3 h and 6 h, and 4 h - 6 h sums share the halved sums of the others;
 //   * constants of the rates and the uniform force come from the host
 //     (StepArgs::k64, the same IEEE operations), not from every thread;
-//   * terms of force components that are zero add zeros, and are left out.
-// Same bits as the plain form; 256^3 TRT cavity 8.93 -> 7.41 ms a step, duct
-// 100x61x47 TRT 162 -> 133 us, channel 4x34x4 BGK 10.7 -> 9.4 us.
+//   * terms of force components that are zero add zeros, and are left out;
+//   * the bulk of the sites (collide_int) does the additions of the moments
+//     and the products with constants on the integer pipes, beside the FP64
+//     pipe.
+// Same bits as the plain form.  128^3 cavity, us a step (plain, fewer FP64
+// operations, with the integer form): TRT 1111, ~925, 559; BGK 938, -, 487;
+// regularized 938, -, 518.  Duct 100x61x47 TRT 161, 133, 89.
 template <int SCH> struct Phys64 : Phys64Base {
     static constexpr bool host_consts = true;
 
@@ -68,20 +72,40 @@ template <int SCH> struct Phys64 : Phys64Base {
         put(9, __fma_rn(-0.5, h[4] + h[7] + h[9], (1.0 / 3.0) * h[0]));
     }
 
+    // relaxed moments of BGK / TRT from den and the stored velocity
+    __device__ static void relaxed_moments(C *h, const Force64 &F, const Consts64 &k, C den, C &ux, C &uy, C &uz) {
+        if (F.mask & 1u) ux = __fma_rn(0.5, F.a[0], ux);
+        if (F.mask & 2u) uy = __fma_rn(0.5, F.a[1], uy);
+        if (F.mask & 4u) uz = __fma_rn(0.5, F.a[2], uz);
+        const C jx = den * ux, jy = den * uy, jz = den * uz;
+        h[0] = den * k.we; h[1] = jx * k.wodd; h[2] = jy * k.wodd; h[3] = jz * k.wodd;
+        h[4] = jx * ux * k.we; h[5] = jx * uy * k.we; h[6] = jx * uz * k.we;
+        h[7] = jy * uy * k.we; h[8] = jy * uz * k.we; h[9] = jz * uz * k.we;
+        force(h, F, k, den, jx, jy, jz);
+    }
+    // regularized: h holds the moments of f; relaxes them and sets the
+    // stored velocity
+    __device__ static void relaxed_moments_reg(C *h, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz) {
+        const C den = h[0], inv = 1.0 / den;
+        C jx = h[1], jy = h[2], jz = h[3];
+        if (F.mask & 1u) jx = __fma_rn(0.5, F.a[0] * den, jx);
+        if (F.mask & 2u) jy = __fma_rn(0.5, F.a[1] * den, jy);
+        if (F.mask & 4u) jz = __fma_rn(0.5, F.a[2] * den, jz);
+        ux = inv * jx; uy = inv * jy; uz = inv * jz;
+        const C ex = den * ux, ey = den * uy, ez = den * uz;
+        const C he[10] = {den, ex, ey, ez, ex * ux, ex * uy, ex * uz, ey * uy, ey * uz, ez * uz};
+#pragma unroll
+        for (int m = 0; m < 10; ++m) h[m] = h[m] * k.r9 + k.we * he[m];
+        force(h, F, k, den, jx, jy, jz);
+    }
+
     // forward-Euler update; returns den, writes the stored velocity
     // u = j/den + a/2 (jyulb/D3Q19.pyx:655-940)
     __device__ static C collide(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz) {
         C h[10];
         if (SCH != SCH_REG) {
             const C den = f_to_den_vel(f, ux, uy, uz);
-            if (F.mask & 1u) ux = __fma_rn(0.5, F.a[0], ux);
-            if (F.mask & 2u) uy = __fma_rn(0.5, F.a[1], uy);
-            if (F.mask & 4u) uz = __fma_rn(0.5, F.a[2], uz);
-            const C jx = den * ux, jy = den * uy, jz = den * uz;
-            h[0] = den * k.we; h[1] = jx * k.wodd; h[2] = jy * k.wodd; h[3] = jz * k.wodd;
-            h[4] = jx * ux * k.we; h[5] = jx * uy * k.we; h[6] = jx * uz * k.we;
-            h[7] = jy * uy * k.we; h[8] = jy * uz * k.we; h[9] = jz * uz * k.we;
-            force(h, F, k, den, jx, jy, jz);
+            relaxed_moments(h, F, k, den, ux, uy, uz);
             if (SCH == SCH_BGK) {
 #pragma unroll
                 for (int q = 0; q < Q; ++q) f[q] = f[q] * k.r9;
@@ -115,20 +139,135 @@ template <int SCH> struct Phys64 : Phys64Base {
             h[7] = (d1y + dy1) - d3;
             h[8] = f[5] + f[13] - f[7] - f[11];
             h[9] = (d1z + dz1) - d3;
-            const C inv = 1.0 / den;
-            C jx = h[1], jy = h[2], jz = h[3];
-            if (F.mask & 1u) jx = __fma_rn(0.5, F.a[0] * den, jx);
-            if (F.mask & 2u) jy = __fma_rn(0.5, F.a[1] * den, jy);
-            if (F.mask & 4u) jz = __fma_rn(0.5, F.a[2] * den, jz);
-            ux = inv * jx; uy = inv * jy; uz = inv * jz;
-            const C ex = den * ux, ey = den * uy, ez = den * uz;
-            const C he[10] = {den, ex, ey, ez, ex * ux, ex * uy, ex * uz, ey * uy, ey * uz, ez * uz};
-#pragma unroll
-            for (int m = 0; m < 10; ++m) h[m] = h[m] * k.r9 + k.we * he[m];
-            force(h, F, k, den, jx, jy, jz);
+            relaxed_moments_reg(h, F, k, ux, uy, uz);
             project_fused<false>(h, f);
             return den;
         }
+    }
+    // the same out of line, for the rare site that collide_int refuses
+    __device__ __noinline__ static C collide_cold(C *f, const Force64 &F, const Consts64 &k, C *u) {
+        return collide(f, F, k, u[0], u[1], u[2]);
+    }
+
+    // The same update, with the additions of the moments and the products with
+    // constants on the integer pipes (soft64.cuh): the same bits.  It needs
+    // populations in [2^-9, 1/4) (rest: up to 1/2) and projections that are
+    // positive; anything else sets `bad` and leaves f undefined.
+    __device__ static C collide_int(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz, bool &bad) {
+        using namespace soft64;
+        C h[10], den;
+        uint32_t range = 0, range9 = 0, least = 0;
+        {
+            uint64_t x[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) x[q] = fix(f[q], q == 9 ? range9 : range);
+            const uint64_t d1x = add(add(add(add(x[0], x[1]), x[2]), x[3]), x[4]);
+            const uint64_t dx1 = add(add(add(add(x[14], x[15]), x[16]), x[17]), x[18]);
+            const uint64_t d01y = add(add(x[5], x[6]), x[7]);
+            const uint64_t d0y1 = add(add(x[11], x[12]), x[13]);
+            const uint64_t xx = add(d1x, dx1);
+            den = to_double(add(add(add(add(add(xx, d01y), d0y1), x[8]), x[9]), x[10]));
+            const C jx = diff_to_double(dx1, d1x);
+            if (SCH != SCH_REG) {
+                // jyulb/D3Q19.pyx:348-390
+                const uint64_t y = sub(sub(add(add(x[4], d0y1), x[18]), x[0], least), d01y, least);
+                const uint64_t zp = add(add(add(add(x[3], x[7]), x[10]), x[13]), x[17]);
+                const uint64_t z = sub(sub(sub(sub(zp, x[1], least), x[5], least), x[8], least), x[11], least);
+                const C jy = diff_to_double(y, x[14]), jz = diff_to_double(z, x[15]);
+                const C inv = 1.0 / den;
+                ux = inv * jx; uy = inv * jy; uz = inv * jz;
+            } else {
+                // jyulb/D3Q19.pyx:395-452
+                const uint64_t d1y = add(add(x[0], d01y), x[14]), dy1 = add(add(x[4], d0y1), x[18]);
+                const uint64_t d1z = add(add(add(add(x[1], x[5]), x[8]), x[11]), x[15]);
+                const uint64_t dz1 = add(add(add(add(x[3], x[7]), x[10]), x[13]), x[17]);
+                const C d3 = (1.0 / 3.0) * den;
+                h[0] = den; h[1] = jx; h[2] = diff_to_double(dy1, d1y); h[3] = diff_to_double(dz1, d1z);
+                h[4] = to_double(xx) - d3;
+                h[5] = diff_to_double(sub(add(x[0], x[18]), x[4], least), x[14]);
+                h[6] = diff_to_double(sub(add(x[1], x[17]), x[3], least), x[15]);
+                h[7] = to_double(add(d1y, dy1)) - d3;
+                h[8] = diff_to_double(sub(add(x[5], x[13]), x[7], least), x[11]);
+                h[9] = to_double(add(d1z, dz1)) - d3;
+            }
+        }
+        if (SCH != SCH_REG) {
+            relaxed_moments(h, F, k, den, ux, uy, uz);
+            if (SCH == SCH_BGK) {
+                // 1 - we = 0 (tau = 1) leaves the projection alone
+                if (k.nonzero & 4u) {
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) f[q] = mul(f[q], k.mr9);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) f[q] = 0.0;
+                }
+            } else {
+                if (!(k.nonzero & 3u)) { // c3 = c4 = 0 (both rates 1)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) if (q != 9) f[q] = 0.0;
+                } else if (!(k.nonzero & 1u)) { // c3 = 0: 0 - c4 f
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) {
+                        const C fa = f[q], fb = f[18 - q];
+                        f[q] = -mul(fb, k.mc4);
+                        f[18 - q] = -mul(fa, k.mc4);
+                    }
+                } else if (!(k.nonzero & 2u)) { // c4 = 0 (equal rates)
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) {
+                        f[q] = mul(f[q], k.mc3);
+                        f[18 - q] = mul(f[18 - q], k.mc3);
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) {
+                        const C fa = f[q], fb = f[18 - q];
+                        f[q] = mul(fa, k.mc3) - mul(fb, k.mc4);
+                        f[18 - q] = mul(fb, k.mc3) - mul(fa, k.mc4);
+                    }
+                }
+                f[9] = k.nonzero & 4u ? mul(f[9], k.mr9) : 0.0;
+            }
+        } else {
+            relaxed_moments_reg(h, F, k, ux, uy, uz);
+        }
+        uint32_t span = 0;
+        project_int<SCH != SCH_REG>(h, k, f, span);
+        bad = range > 6u || range9 > 7u || least >= (1u << 31) - (1u << 21) || span > PROJ_SPAN;
+        return den;
+    }
+
+    // project_fused with integer products; `span` exceeds PROJ_SPAN unless
+    // every projection argument lies in [2^-40, 2^10)
+    static constexpr uint32_t PROJ_LO = (1023u - 40u) << 20, PROJ_SPAN = (50u << 20) - 1u;
+    template <bool ADD> __device__ static void project_int(const C *h, const Consts64 &k, C *f, uint32_t &span) {
+        const C t4 = 3.0 * h[4], t7 = 3.0 * h[7], t9 = 3.0 * h[9];
+        const C s = h[0] + t4, v = __fma_rn(2.0, h[0], -t4);
+        const C w = __fma_rn(2.0, s, -t7), v2 = __fma_rn(2.0, t7, v);
+        const C exy = __fma_rn(2.0, s + t7, -t9), exz = __fma_rn(2.0, t9, w), eyz = __fma_rn(2.0, t9, v2);
+        const C ex = w - t9, ey = v2 - t9, ez = __fma_rn(2.0, t9, v - t7);
+        const C q1 = 6.0 * h[1], q2 = 6.0 * h[2], q3 = 6.0 * h[3];
+        auto scaled = [&](C y, const soft64::MulC &m) {
+            const uint32_t e = (uint32_t)__double2hiint(y) - PROJ_LO;
+            span = span > e ? span : e;
+            return soft64::mul(y, m);
+        };
+        auto put = [&](int q, C p) { f[q] = ADD ? f[q] + p : p; };
+        auto pair = [&](int lo, C e, C o) {
+            put(lo, scaled(e - o, k.m72));
+            put(18 - lo, scaled(e + o, k.m72));
+        };
+        auto axis = [&](int lo, C e, C o) {
+            put(lo, scaled(e - o, k.m36));
+            put(18 - lo, scaled(e + o, k.m36));
+        };
+        C o;
+        o = 18.0 * h[5]; pair(0, exy + o, q1 + q2); pair(4, exy - o, q1 - q2);
+        o = 18.0 * h[6]; pair(1, exz + o, q1 + q3); pair(3, exz - o, q1 - q3);
+        o = 18.0 * h[8]; pair(5, eyz + o, q2 + q3); pair(7, eyz - o, q2 - q3);
+        axis(2, ex, q1); axis(6, ey, q2); axis(8, ez, q3);
+        put(9, __fma_rn(-0.5, h[4] + h[7] + h[9], (1.0 / 3.0) * h[0]));
     }
 };
 

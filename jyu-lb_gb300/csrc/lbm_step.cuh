@@ -242,7 +242,8 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
 
     // gather: a bounce-back link reads its own opposite slot; the choice is a
     // select, not a branch
-    Unroll<0, Q>::run([&]<int q>() {
+    auto gather = [&](C *g) {
+      Unroll<0, Q>::run([&]<int q>() {
         IT e;
         if (!PSTEP || q == 9) {
             e = (IT)q * Np + n;
@@ -252,8 +253,10 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
             const IT e_bb = (IT)q * Np + n;
             e = (m & (1u << q)) ? e_bb : e_reg;
         }
-        fv[q] = bulk_ld<ST, PH, q>(f + e);
-    });
+        g[q] = bulk_ld<ST, PH, q>(f + e);
+      });
+    };
+    gather(fv);
 
     C ux, uy, uz, rho;
     if constexpr (uses_force_density<PH>::value) {
@@ -265,7 +268,18 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
         rho = PH::collide_fd(fv, arg_g<C>(a, 0), arg_g<C>(a, 1), arg_g<C>(a, 2), fx, fy, fz, arg_we<C>(a),
                              arg_wo<C>(a), ux, uy, uz);
     } else if constexpr (uses_host_consts<PH>::value) {
-        rho = PH::collide(fv, site_force64<ACCF>(a, n), a.k64, ux, uy, uz);
+        const Force64 F = site_force64<ACCF>(a, n);
+        bool bad = true;
+        if (a.k64.soft) rho = PH::collide_int(fv, F, a.k64, ux, uy, uz, bad);
+        if (bad) {
+            // outside the integer form's range: nothing is stored yet, so the
+            // site is read again and takes the FP64 form
+            C g[Q], u[3];
+            gather(g);
+            rho = PH::collide_cold(g, F, a.k64, u);
+            ux = u[0]; uy = u[1]; uz = u[2];
+            Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
+        }
     } else {
         C ax, ay, az;
         if (ACCF) {

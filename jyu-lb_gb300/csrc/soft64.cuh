@@ -1,0 +1,186 @@
+// soft64.cuh -- correctly rounded FP64 operations on the integer pipes.
+//
+// GB300 issues one FP64 warp instruction per 19 cycles and SM, but two integer
+// (ALU) warp instructions and two 32x32->64 multiply-adds per cycle.  An
+// FP64 product with a constant takes 16 integer instructions and 4
+// multiply-adds here (8 cycles), one addition of a chain of positive numbers
+// in fixed point 11 (5.5 cycles), and both run beside the FP64 pipe.  Every
+// function returns the bits that the IEEE operation with rounding to nearest
+// even returns, on the operand ranges stated; callers check those ranges and
+// take the plain operations otherwise.  The arithmetic follows IEEE 754 from
+// its definition (exact product or sum, then one rounding) and runs on the
+// host too, where the tests compare it with the hardware.
+#pragma once
+#include <stdint.h>
+#include <string.h>
+
+#include <cuda_runtime.h>
+
+namespace jlb {
+namespace soft64 {
+
+#if defined(__CUDACC__)
+#define S64_FN __host__ __device__ __forceinline__
+#else
+#define S64_FN inline
+#endif
+
+S64_FN uint64_t bits(double x) {
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return u;
+#endif
+}
+S64_FN double from(uint32_t hi, uint32_t lo) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double((int)hi, (int)lo);
+#else
+    const uint64_t u = ((uint64_t)hi << 32) | lo;
+    double x;
+    memcpy(&x, &u, 8);
+    return x;
+#endif
+}
+// index of the highest set bit (of a nonzero word; 0xffffffff for 0)
+S64_FN uint32_t top_bit(uint32_t x) {
+#ifdef __CUDA_ARCH__
+    uint32_t r;
+    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+#else
+    return x ? 31u - (uint32_t)__builtin_clz(x) : 0xffffffffu;
+#endif
+}
+// the n low bits set, 0 <= n <= 31
+S64_FN uint32_t low_mask(uint32_t n) {
+#ifdef __CUDA_ARCH__
+    uint32_t r;
+    asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(r) : "r"(n));
+    return r;
+#else
+    return (1u << n) - 1u;
+#endif
+}
+// high word of (hi:lo) << s, 0 <= s <= 31
+S64_FN uint32_t shl_hi(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, s);
+#else
+    return s ? (hi << s) | (lo >> (32 - s)) : hi;
+#endif
+}
+// low word of (hi:lo) >> s, 0 <= s <= 31
+S64_FN uint32_t shr_lo(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, s);
+#else
+    return s ? (lo >> s) | (hi << (32 - s)) : lo;
+#endif
+}
+
+// A nonzero normal constant k prepared for mul(): its 53-bit significand
+// shifted to [2^61, 2^62), and what its exponent and sign add to the high word
+struct MulC {
+    uint32_t hi, lo, base;
+};
+inline MulC make_mulc(double k) {
+    const uint64_t u = bits(k);
+    const uint64_t m = ((u & 0xfffffffffffffull) | (1ull << 52)) << 9;
+    const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+    return MulC{(uint32_t)(m >> 32), (uint32_t)m, ((e - 1024u) << 20) ^ (uint32_t)((u >> 63) << 31)};
+}
+
+// x * k for normal x with a normal product.  The 115-bit product's leading
+// bits are shifted to 53; what is left out is one word with a sticky bit, into
+// which the last kept bit goes too, so that "more than half" decides ties to
+// even
+S64_FN double mul(double x, const MulC &k) {
+    const uint64_t u = bits(x);
+    const uint32_t xh = (uint32_t)(u >> 32), l = (uint32_t)u;
+    const uint32_t h = (xh & 0xfffffu) | 0x100000u;
+    const uint64_t t0 = (uint64_t)l * k.lo;
+    const uint64_t t1 = (uint64_t)h * k.lo + (t0 >> 32);
+    const uint64_t t2 = (uint64_t)l * k.hi + t1;
+    const uint64_t t3 = (uint64_t)h * k.hi + (t2 >> 32); // [2^49, 2^51)
+    const uint32_t th = (uint32_t)(t3 >> 32), tl = (uint32_t)t3, w = (uint32_t)t2;
+    const uint32_t c = th >> 18, s = 3u - c;
+    const uint32_t ml = shl_hi(w, tl, s), mh = shl_hi(tl, th, s);
+    const uint32_t low = (uint32_t)t0;
+    const uint32_t sticky = low < 1u ? low : 1u;
+    const uint32_t rest = (w << s) | ((sticky | ml) & 1u);
+    const uint64_t up = ((uint64_t)rest + 0x7fffffffu) >> 32;
+    const uint64_t m = (((uint64_t)mh << 32) | ml) + up;
+    return from((uint32_t)(m >> 32) + (xh & 0xfff00000u) + k.base + (c << 20), (uint32_t)m);
+}
+
+// ---------------------------------------------------------------------------
+// Chains of additions in fixed point with unit 2^-61.  Each add() rounds as
+// the FP64 addition does: to 53 significant bits of the partial sum.
+// ---------------------------------------------------------------------------
+constexpr uint32_t FIX_E0 = 1014; // exponent field of 2^-9, the least operand
+
+// x in [2^-9, 2^(n-9)) as fixed point; `range` collects field - 1014, which is
+// n or more for anything else (negative numbers, zeros, infinities, NaN)
+S64_FN uint64_t fix(double x, uint32_t &range) {
+    const uint64_t u = bits(x);
+    const uint32_t xh = (uint32_t)(u >> 32), xl = (uint32_t)u;
+    const uint32_t s = (xh >> 20) - FIX_E0;
+    range = range > s ? range : s;
+    const uint32_t h = (xh & 0xfffffu) | 0x100000u;
+#ifdef __CUDA_ARCH__
+    return ((uint64_t)shl_hi(xl, h, s) << 32) | (uint32_t)(xl << (s & 31u));
+#else
+    return ((uint64_t)shl_hi(xl, h, s & 31u) << 32) | (uint32_t)(xl << (s & 31u));
+#endif
+}
+
+// a + b for positive operands (the sum is at least 2^53 units)
+S64_FN uint64_t add(uint64_t a, uint64_t b) {
+    const uint64_t s = a + b;
+    const uint32_t hi = (uint32_t)(s >> 32), lo = (uint32_t)s;
+    const uint32_t d = top_bit(hi) - 20u;
+    const uint32_t mask = low_mask(d);
+    const uint32_t odd = (lo >> d) & 1u;
+    return (s + ((mask >> 1) + odd)) & ~(uint64_t)mask;
+}
+// a - b, expected positive and at least 2^53 units (checked through p; a
+// negative difference has its top bit set, which the check sees as hi >= 2^31)
+S64_FN uint64_t sub(uint64_t a, uint64_t b, uint32_t &p) {
+    const uint64_t s = a - b;
+    const uint32_t hi = (uint32_t)(s >> 32);
+    const uint32_t q = hi - (1u << 21);
+    p = p > q ? p : q; // below 2^31 - 2^21 for sums in range
+    return add(s, 0);
+}
+
+// a fixed-point number already rounded to 53 bits, as a double
+S64_FN double to_double(uint64_t s) {
+    const uint32_t hi = (uint32_t)(s >> 32), lo = (uint32_t)s;
+    const uint32_t d = top_bit(hi) - 20u;
+    return from((hi >> d) + ((d + FIX_E0 - 1u) << 20), shr_lo(lo, hi, d));
+}
+// the signed difference a - b (|a - b| < 2^63 units) rounded to a double; an
+// exact zero is +0 as in IEEE subtraction
+S64_FN double diff_to_double(uint64_t a, uint64_t b) {
+    const uint64_t s = a - b;
+    const uint32_t sign = (uint32_t)(s >> 63);
+    const uint64_t m = (s ^ (0ull - sign)) + sign;
+    uint32_t hi = (uint32_t)(m >> 32), lo = (uint32_t)m, e = 1014u + 10u + 1u;
+    // leading bit to bit 63
+    if (hi == 0) { hi = lo; lo = 0; e -= 32u; }
+    const uint32_t z = 31u - top_bit(hi); // 32 for zero
+    const uint32_t nh = shl_hi(lo, hi, z & 31u), nl = lo << (z & 31u);
+    // 53 of 64 bits stay
+    const uint32_t ml = shr_lo(nl, nh, 11u), mh = nh >> 11;
+    const uint32_t rest = (nl << 21) | (ml & 1u);
+    const uint64_t up = ((uint64_t)rest + 0x7fffffffu) >> 32;
+    const uint64_t r = (((uint64_t)mh << 32) | ml) + up;
+    const uint32_t rh = (uint32_t)(r >> 32) + ((e - 1u - z) << 20) + (sign << 31);
+    return hi == 0 ? 0.0 : from(rh, (uint32_t)r);
+}
+
+} // namespace soft64
+} // namespace jlb
