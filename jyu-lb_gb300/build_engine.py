@@ -27,8 +27,10 @@ UNITS = {
     # work for different warps at once.  128^3 TRT cavity 671 / 591 / 559 /
     # 570 us a step at 2 / 3 / 4 / 5
     "lbm_fp64.cu": ["-fmad=false", "-DJLB_MIN_BLOCKS=4"],
-    # the fast FP64 step: contracted on purpose
-    "lbm_fp64fast.cu": [],
+    # the fast FP64 step: contracted on purpose.  5 resident blocks (96
+    # registers, a few spilled): 256^3 TRT cavity 1390 / 1197 / 1178 us a step
+    # at 3 / 4 / 5
+    "lbm_fp64fast.cu": ["-DJLB_MIN_BLOCKS=5"],
     # resident 128-thread blocks per SM.  The direct steps are latency-bound
     # on HBM: 8 blocks (<= 64 registers, 32 warps) keep more loads in flight
     # than 6 or 7, even where a few registers spill.  The persistent staged L
@@ -50,7 +52,7 @@ UNITS = {
     "lbm_batch_host.cpp": HOST_FLAGS,
     "lbm_adjoint_host.cpp": HOST_FLAGS,
 }
-HEADERS = ["lbm_common.h", "soft64.cuh", "lbm_fp64.cuh", "lbm_solver.h", "lbm_step.cuh", "lbm_step_tma.cuh", "lbm_shifted.cuh", "lbm_aux.h", "lbm_batch.h", "lbm_adjoint.h"]
+HEADERS = ["lbm_common.h", "soft64.cuh", "lbm_fixed64.cuh", "lbm_fp64.cuh", "lbm_solver.h", "lbm_step.cuh", "lbm_step_tma.cuh", "lbm_shifted.cuh", "lbm_aux.h", "lbm_batch.h", "lbm_adjoint.h"]
 
 
 def _nvcc() -> str:

@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cuda_runtime.h>
 
+#include "lbm_fixed64.cuh"
 #include "soft64.cuh"
 
 namespace jlb {
@@ -134,6 +135,7 @@ struct StepArgs {
     Consts64 k64;         // FP64 collision constants
     double c1;            // first-moment force factor: 1 - wo/2 (TRT), 1 - we/2
     Force64 g64;          // uniform gravity with its factors
+    FixConsts fx;         // constants of the fixed-point collision (JLB_FP64_FAST)
     int write_moments;
     // dense-node grid
     int bx, by, kblocks;  // block shape and k-blocks per row-block
@@ -192,6 +194,7 @@ inline void set_consts64(StepArgs &a, int scheme) {
         if (rel[i] != 0.0) k.nonzero |= 1u << i;
         if (rel[i] != 0.0 && !(std::fabs(rel[i]) > 0x1p-200 && std::fabs(rel[i]) < 0x1p10)) k.soft = 0;
     }
+    a.fx = make_fix_consts(scheme == SCH_TRT, scheme == SCH_REG, a.w_e, a.w_o, a.g);
     // the regularized update weighs the first-moment force by 1 - we/2 too
     a.c1 = scheme == SCH_TRT ? 1.0 - 0.5 * a.w_o : k.c2;
     a.g64.mask = 0;

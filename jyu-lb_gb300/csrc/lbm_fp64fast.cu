@@ -4,16 +4,19 @@
 // Same storage, layout, boundary handling and physics as the parity step
 // (lbm_fp64.cu): BGK / TRT / regularized collision of the reference
 // (jyulb/D3Q19.pyx:655-940) with its forcing and stored velocity
-// u = j/den + a/2.  The arithmetic is reorganised for GB300, whose FP64 rate
-// (not HBM) bounds the parity step at ~276 separately rounded operations per
-// TRT site:
+// u = j/den + a/2.  The bulk of the sites collides in 64-bit fixed point
+// (lbm_fixed64.cuh), which GB300's integer pipes do several times faster than
+// its FP64 pipe does FP64 and which loses less: 256^3 TRT cavity 5497 -> 1178
+// us a step, 128^3 699 -> 166, 40x33x27 15.2 -> 6.0.  Boundary nodes, sites
+// with an acceleration field and sites outside the fixed-point range take the
+// FP64 form below:
 //   * den, j and u in the reference's order and rounding,
 //   * the projection of the H10 moments grouped per pair of opposite
 //     populations (even part e, odd part o) and merged with the TRT pair
 //     relaxation: f_q <- fma(c3, f_q, fma(-c4, f_opp, e + o)),
 //   * den u formed as j + den a/2 directly,
-// and the unit is compiled with FMA contraction.  Boundary nodes use the
-// reference's Zou-He and Ladd expressions (lbm_fp64.cuh), contracted.
+// compiled with FMA contraction; their Zou-He and Ladd expressions are the
+// reference's (lbm_fp64.cuh), contracted.
 // Results differ from the parity step by rounding only: within 1e-12
 // relative of the reference on every golden case, at up to 1000 steps.
 #include "lbm_fp64.cuh"
@@ -79,6 +82,14 @@ struct Phys64FBase : Phys64Base {
 };
 
 template <int SCH> struct Phys64F : Phys64FBase {
+    // the bulk of the sites without an acceleration field
+    static constexpr bool fixed_point = true, regularized = SCH == SCH_REG;
+
+    // out of line, for the rare site the fixed-point form refuses
+    __device__ __noinline__ static void collide_cold(C *f, const double *g, C we, C wo, C *mom) {
+        mom[0] = collide(f, g[0], g[1], g[2], we, wo, mom[1], mom[2], mom[3]);
+    }
+
     // returns den, writes the stored velocity u = j/den + a/2
     __device__ static C collide(C *f, C ax, C ay, C az, C we, C wo, C &ux, C &uy, C &uz) {
         C jx, jy, jz;

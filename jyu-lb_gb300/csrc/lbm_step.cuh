@@ -149,6 +149,14 @@ template <class PH, class = void> struct uses_host_consts {
 template <class PH> struct uses_host_consts<PH, std::void_t<decltype(PH::host_consts)>> {
     static constexpr bool value = PH::host_consts;
 };
+// physics policies whose bulk sites collide in fixed point (lbm_fixed64.cuh)
+// declare fixed_point = true
+template <class PH, class = void> struct uses_fixed_point {
+    static constexpr bool value = false;
+};
+template <class PH> struct uses_fixed_point<PH, std::void_t<decltype(PH::fixed_point)>> {
+    static constexpr bool value = PH::fixed_point;
+};
 // the force of site n: the uniform one with the host's factors, or with the
 // acceleration field added (its factors are formed here, in the same order)
 template <bool ACCF> __device__ __forceinline__ Force64 site_force64(const StepArgs &a, int64_t n) {
@@ -280,6 +288,19 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
             ux = u[0]; uy = u[1]; uz = u[2];
             Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
         }
+    } else if constexpr (uses_fixed_point<PH>::value && !ACCF) {
+        C mom[4];
+        bool good = false;
+        if (a.fx.ok) good = collide_fixed<PH::regularized>(fv, a.fx, a.g, a.write_moments != 0, mom);
+        if (!good) {
+            // outside the fixed-point range: the site is read again and takes
+            // the FP64 form
+            C g[Q];
+            gather(g);
+            PH::collide_cold(g, a.g, a.w_e, a.w_o, mom);
+            Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
+        }
+        rho = mom[0]; ux = mom[1]; uy = mom[2]; uz = mom[3];
     } else {
         C ax, ay, az;
         if (ACCF) {

@@ -130,11 +130,7 @@ S64_FN uint64_t fix(double x, uint32_t &range) {
     const uint32_t s = (xh >> 20) - FIX_E0;
     range = range > s ? range : s;
     const uint32_t h = (xh & 0xfffffu) | 0x100000u;
-#ifdef __CUDA_ARCH__
-    return ((uint64_t)shl_hi(xl, h, s) << 32) | (uint32_t)(xl << (s & 31u));
-#else
     return ((uint64_t)shl_hi(xl, h, s & 31u) << 32) | (uint32_t)(xl << (s & 31u));
-#endif
 }
 
 // a + b for positive operands (the sum is at least 2^53 units)
@@ -180,6 +176,55 @@ S64_FN double diff_to_double(uint64_t a, uint64_t b) {
     const uint64_t r = (((uint64_t)mh << 32) | ml) + up;
     const uint32_t rh = (uint32_t)(r >> 32) + ((e - 1u - z) << 20) + (sign << 31);
     return hi == 0 ? 0.0 : from(rh, (uint32_t)r);
+}
+
+// ---------------------------------------------------------------------------
+// Signed fixed-point products.  A 64-bit number is split into balanced 32-bit
+// digits (low digit in [-2^31, 2^31)), so that three signed 32x32->64
+// multiply-adds give the product's high half; the product of the two low
+// digits, at most a quarter of the last place and zero on average, is left out.
+// ---------------------------------------------------------------------------
+struct Fix2 {
+    int32_t hi, lo;
+};
+S64_FN Fix2 digits(int64_t x) {
+    Fix2 d;
+    d.lo = (int32_t)(uint32_t)(uint64_t)x;
+    d.hi = (int32_t)((x + 0x80000000ll) >> 32);
+    return d;
+}
+// x y / 2^(64 - SH), rounded; |x| < 2^62, |y| < 2^62 and no overflow of the
+// result
+template <int SH = 0> S64_FN int64_t mulq(const Fix2 &x, const Fix2 &y) {
+    int64_t m = (int64_t)x.lo * y.hi + (0x80000000ll >> SH);
+    m = (int64_t)x.hi * y.lo + m;
+    return (int64_t)x.hi * y.hi * (1ll << SH) + (m >> (32 - SH));
+}
+template <int SH = 0> S64_FN int64_t mulq(int64_t x, const Fix2 &y) { return mulq<SH>(digits(x), y); }
+
+// a positive number of 53 to 63 bits (unit 2^-61) rounded to a double;
+// `low` collects what makes it 2^31 - 2^20 or more for any other number
+S64_FN double round_to_double(int64_t v, uint32_t &low) {
+    uint64_t s = (uint64_t)v;
+    uint32_t hi = (uint32_t)(s >> 32);
+    const uint32_t c = hi - (1u << 20);
+    low = low > c ? low : c;
+    const uint32_t d = (top_bit(hi) - 20u) & 31u;
+    const uint32_t mask = low_mask(d), lo = (uint32_t)s;
+    const uint32_t odd = (lo >> d) & mask & 1u;
+    s = s + ((mask >> 1) + odd);
+    hi = (uint32_t)(s >> 32);
+    // bits below the last kept one go with the shift; a carry into the next
+    // binade moves the exponent
+    return from((hi >> d) + ((d + FIX_E0 - 1u) << 20), shr_lo((uint32_t)s, hi, d));
+}
+// a positive double in [2^-1, 2) with unit 2^-62
+S64_FN int64_t fix62(double x) {
+    const uint64_t u = bits(x);
+    const uint32_t xh = (uint32_t)(u >> 32), xl = (uint32_t)u;
+    const uint32_t s = ((xh >> 20) - (FIX_E0 - 1u)) & 31u;
+    const uint32_t h = (xh & 0xfffffu) | 0x100000u;
+    return (int64_t)(((uint64_t)shl_hi(xl, h, s) << 32) | (uint32_t)(xl << s));
 }
 
 } // namespace soft64
