@@ -504,13 +504,17 @@ __device__ __forceinline__ void adjoint_boundary_sites(const AdjArgs &A, int b, 
 
 int adjoint_blocks(const StepArgs &a) { return a.nb_dense + special_blocks(a); }
 
-// One step of the reverse sweep: blocks [0, nb_dense) take the dense sites,
-// the rest the boundary sites (disjoint address sets, as in the forward step).
+// One step of the reverse sweep: the first blocks take the boundary sites,
+// the last nb_dense the dense sites (disjoint address sets, as in the forward step).
 template <class ST, int SCH, bool PSTEP, bool SEED, class IT>
 __global__ void __launch_bounds__(128, adj_min_blocks<ST, SEED>()) adjoint_step_kernel(const AdjArgs A) {
     using C = typename ST::C;
     C pg[5] = {0, 0, 0, 0, 0};
-    const int b = (int)blockIdx.x;
+    // boundary sites first (the longer chain); a block's slot does not depend
+    // on the launch order: dense blocks, then boundary blocks
+    const int nsp = (int)gridDim.x - A.s.nb_dense;
+    const int n = (int)blockIdx.x - nsp;
+    const int b = n < 0 ? A.s.nb_dense + (int)blockIdx.x : n;
     if (b < A.s.nb_dense) adjoint_dense_sites<ST, SCH, PSTEP, SEED, IT>(A, b, pg);
     else adjoint_boundary_sites<ST, SCH, PSTEP, SEED>(A, b - A.s.nb_dense, pg);
     block_sensitivities<C>(pg, A.part + 5 * (int64_t)b);

@@ -2,10 +2,10 @@
 // collide + moments) for one AA half-pair, generic over the storage policy
 // and the collision physics.
 //
-// One launch per time step.  Blocks [0, nb_dense) sweep the lattice in
+// One launch per time step.  The last nb_dense blocks sweep the lattice in
 // (k-fastest) rows: every fluid node that is not a boundary node streams with
 // plain neighbour arithmetic (periodic wrap for free) and halfway bounce-back
-// from its 19-bit link mask.  Blocks [nb_dense, grid) handle the boundary
+// from its 19-bit link mask.  The blocks before them handle the boundary
 // nodes from a precomputed list: Zou-He faces, links that cross a symmetric
 // face, and links to moving solids (Ladd's term), each with explicit per-link
 // read/write element indices.  The two sets are disjoint and the AA pattern
@@ -363,6 +363,7 @@ __device__ __forceinline__ void special_node(const StepArgs &a, int b) {
     const C dprev = spden[t];
     C fv[Q];
 
+    const uint32_t faces = (info >> SP_FACE_SHIFT) & 0x3Fu;
     Unroll<0, Q>::run([&]<int q>() {
         const int64_t addr = PSTEP ? __ldg(a.sp_rd + (int64_t)q * M + t) : (int64_t)q * PNp + pn;
         // the value read may belong to any slot; decode with the slot of q's
@@ -373,7 +374,6 @@ __device__ __forceinline__ void special_node(const StepArgs &a, int b) {
         fv[q] = v;
     });
 
-    const uint32_t faces = (info >> SP_FACE_SHIFT) & 0x3Fu;
     if (faces) {
         int slot = 0;
 #pragma unroll
@@ -400,6 +400,8 @@ __device__ __forceinline__ void special_node(const StepArgs &a, int b) {
         rho = PH::collide_fd(fv, arg_g<C>(a, 0), arg_g<C>(a, 1), arg_g<C>(a, 2), fx, fy, fz, arg_we<C>(a),
                              arg_wo<C>(a), ux, uy, uz);
     } else if constexpr (uses_host_consts<PH>::value) {
+        // the FP64 form: a lid's edge nodes leave the integer form's range, and
+        // a warp that takes both pays for both (9x8x8 cavity 15.5 -> 33.0 us)
         rho = PH::collide(fv, site_force64<ACCF>(a, n), a.k64, ux, uy, uz);
     } else {
         C ax, ay, az;
@@ -580,23 +582,27 @@ __device__ __forceinline__ void prefetch_block(const StepArgs &a, int b, int lan
 #endif
 template <class ST, class PH, bool PSTEP, bool ACCF, class IT>
 __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_STEP) lbm_step_kernel(const StepArgs a) {
-    const int b = (int)blockIdx.x;
-    if (b < a.nb_dense) {
+    // boundary nodes first: their chain of index loads, Zou-He sums and
+    // collision is the longest, and at the end of the grid it was a tail (us a
+    // step, last / first: FP32 duct 200x90x75 36.6 / 32.6, FP32 cavity 60x57x56
+    // 7.6 / 5.6, FP64 duct 100x61x47 88.6 / 79.5, fast FP64 cavity 128^3 166 / 150)
+    const int b = (int)blockIdx.x - ((int)gridDim.x - a.nb_dense);
+    if (b >= 0) {
         if (a.pf && threadIdx.y == 0 && threadIdx.x < 32 && b + a.pf < a.nb_dense)
             prefetch_block<typename ST::S, PSTEP>(a, b + a.pf + a.b0, (int)threadIdx.x);
         dense_node<ST, PH, PSTEP, ACCF, IT>(a, b + a.b0);
     } else {
-        special_node<ST, PH, PSTEP, ACCF>(a, b - a.nb_dense);
+        special_node<ST, PH, PSTEP, ACCF>(a, (int)blockIdx.x);
     }
 }
 
 template <class ST, class PH, bool PSTEP, bool ACCF>
 __global__ void __launch_bounds__(128, PSTEP ? JLB_MIN_BLOCKS_SPARSE : JLB_MIN_BLOCKS_SPARSE_L)
     lbm_step_sparse_kernel(const StepArgs a) {
-    const int b = (int)blockIdx.x;
     const int nbc = (int)((a.Nc + 127) / 128);
-    if (b < nbc) sparse_node<ST, PH, PSTEP, ACCF>(a, b);
-    else special_node<ST, PH, PSTEP, ACCF>(a, b - nbc);
+    const int b = (int)blockIdx.x - ((int)gridDim.x - nbc); // boundary nodes first
+    if (b >= 0) sparse_node<ST, PH, PSTEP, ACCF>(a, b);
+    else special_node<ST, PH, PSTEP, ACCF>(a, (int)blockIdx.x);
 }
 
 template <class ST, template <int> class PH>

@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_TMA) lbm_step_tma_kernel(c
     int tile = blockIdx.x;
     int it = 0;
     if (tile < ntiles && t == 0) tma_issue<S, PSTEP>(a, tile, buf0, &bar[0]);
+    // boundary nodes while the first tile arrives
+    for (int sb = blockIdx.x; sb < nspecial_blocks; sb += gridDim.x) special_node<ST, PH, PSTEP, ACCF>(a, sb);
     for (; tile < ntiles; tile += gridDim.x, ++it) {
         S *cur = (it & 1) ? buf1 : buf0;
         const int next = tile + gridDim.x;
@@ -224,8 +226,6 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_TMA) lbm_step_tma_kernel(c
         }
         __syncthreads(); // buffer `cur` is free for the copies issued next round
     }
-    // boundary nodes after the tiles
-    for (int sb = blockIdx.x; sb < nspecial_blocks; sb += gridDim.x) special_node<ST, PH, PSTEP, ACCF>(a, sb);
 }
 
 // ---------------------------------------------------------------------------
@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_H2) lbm_step_tma_h2_kernel
     int tile = blockIdx.x;
     int it = 0;
     if (tile < ntiles && t == 0) h2_issue(a, tile, kb2, buf0, &bar[0]);
+    for (int sb = blockIdx.x; sb < nspecial_blocks; sb += gridDim.x) special_node<StoreF16, PH, false, ACCF>(a, sb);
     for (; tile < ntiles; tile += gridDim.x, ++it) {
         const __half *cur = (it & 1) ? buf1 : buf0;
         const int next = tile + gridDim.x;
@@ -344,7 +345,6 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_H2) lbm_step_tma_h2_kernel
         }
         __syncthreads(); // buffer `cur` is free for the copies issued next round
     }
-    for (int sb = blockIdx.x; sb < nspecial_blocks; sb += gridDim.x) special_node<StoreF16, PH, false, ACCF>(a, sb);
 }
 
 template <template <int> class PH>
