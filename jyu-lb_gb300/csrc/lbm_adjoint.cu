@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(128, adj_min_blocks<ST, SEED>()) adjoint_step_
     // on the launch order: dense blocks, then boundary blocks
     const int nsp = (int)gridDim.x - A.s.nb_dense;
     const int n = (int)blockIdx.x - nsp;
-    const int b = n < 0 ? A.s.nb_dense + (int)blockIdx.x : n;
+    const int b = n < 0 ? A.s.nb_dense + (int)blockIdx.x : A.s.rev ? A.s.nb_dense - 1 - n : n;
     if (b < A.s.nb_dense) adjoint_dense_sites<ST, SCH, PSTEP, SEED, IT>(A, b, pg);
     else adjoint_boundary_sites<ST, SCH, PSTEP, SEED>(A, b - A.s.nb_dense, pg);
     block_sensitivities<C>(pg, A.part + 5 * (int64_t)b);

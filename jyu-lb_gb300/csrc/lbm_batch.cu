@@ -50,8 +50,10 @@ __global__ void __launch_bounds__(BLOCK, JLB_BATCH_WARPS * 32 / BLOCK)
     using ST = StoreF32;
     using PH = PhysSh<SCH>;
     using C = float;
-    const int t = (int)blockIdx.x;
-    if (a.pf && threadIdx.x < 32 && t + a.pf < a.ntiles) batch_prefetch<PSTEP, BLOCK>(a, t + a.pf, (int)threadIdx.x);
+    const int b = (int)blockIdx.x;
+    const int t = a.rev ? a.ntiles - 1 - b : b;
+    if (a.pf && threadIdx.x < 32 && b + a.pf < a.ntiles)
+        batch_prefetch<PSTEP, BLOCK>(a, a.rev ? t - a.pf : t + a.pf, (int)threadIdx.x);
     const int d = __ldg(a.tile_dom + t);
     const BatchDomain &D = a.dom[d];
     const int32_t l = (t - D.first_tile) * BLOCK + (int)threadIdx.x;

@@ -39,6 +39,7 @@ struct BatchArgs {
     float *den, *ux, *uy, *uz;
     int write_moments;
     int ntiles;            // tiles of the launch
+    int rev;               // 1: tiles run from the last to the first
     int pf;                // L2 prefetch distance in tiles: the block of tile t
                            // prefetches the rows tile t + pf reads (0: none)
     // boundary nodes of the domains with Zou-He or symmetric faces, in the

@@ -130,7 +130,10 @@ int batch_tiles(jlb_batch *b, int block) {
 }
 
 int batch_launch(jlb_batch *b, bool pstep, int write_moments) {
-    const BatchArgs a = batch_args(b, write_moments);
+    BatchArgs a = batch_args(b, write_moments);
+    // from the end where the last step left its lines in the L2: 32 channels
+    // (0.9 GB) 254.7 -> 248.2 us a step
+    a.rev = !pstep;
     int r = launch_batch_step(a, b->scheme, pstep, b->block, b->ntiles, b->st);
     if (r) return bfail(b, JLB_ERR_CUDA, std::string("batch step: ") + cudaGetErrorString((cudaError_t)r));
     ++b->launches;

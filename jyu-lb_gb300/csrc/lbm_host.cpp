@@ -656,7 +656,15 @@ StepArgs make_args(const jlb_solver *s, int write_moments) {
     return a;
 }
 
-int launch_one(jlb_solver *s, const StepArgs &a, bool pstep) {
+int launch_one(jlb_solver *s, const StepArgs &a0, bool pstep) {
+    StepArgs a = a0;
+    // steps sweep up and down in turn: a step then begins with the lines the
+    // one before left in the L2 (129 MB).  FP32, us a step, one way / both
+    // ways: duct 200x90x75 (103 MB) 32.6 / 27.7, cavity 128^3 (159 MB) 58.6 /
+    // 50.2, porous 192x128x128 (144 MB) 62.2 / 51.7, porous 384x256x256
+    // (1.15 GB) 459 / 450, cavity 256^3 (1.27 GB) 415 / 410; nothing lost where
+    // everything fits (60x57x56: 5.4 / 5.4)
+    a.rev = !pstep;
     const int blocks = a.nb_dense + special_blocks(a); // direct kernel: blocks of bx * by threads
     const int nsb = (a.M + 127) / 128;                  // staged / fluid-only kernels: 128
     int r;

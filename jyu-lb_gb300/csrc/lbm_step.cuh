@@ -588,9 +588,10 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_STEP) lbm_step_kernel(cons
     // 7.6 / 5.6, FP64 duct 100x61x47 88.6 / 79.5, fast FP64 cavity 128^3 166 / 150)
     const int b = (int)blockIdx.x - ((int)gridDim.x - a.nb_dense);
     if (b >= 0) {
+        auto place = [&](int n) { return a.b0 + (a.rev ? a.nb_dense - 1 - n : n); };
         if (a.pf && threadIdx.y == 0 && threadIdx.x < 32 && b + a.pf < a.nb_dense)
-            prefetch_block<typename ST::S, PSTEP>(a, b + a.pf + a.b0, (int)threadIdx.x);
-        dense_node<ST, PH, PSTEP, ACCF, IT>(a, b + a.b0);
+            prefetch_block<typename ST::S, PSTEP>(a, place(b + a.pf), (int)threadIdx.x);
+        dense_node<ST, PH, PSTEP, ACCF, IT>(a, place(b));
     } else {
         special_node<ST, PH, PSTEP, ACCF>(a, (int)blockIdx.x);
     }
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(128, PSTEP ? JLB_MIN_BLOCKS_SPARSE : JLB_MIN_B
     lbm_step_sparse_kernel(const StepArgs a) {
     const int nbc = (int)((a.Nc + 127) / 128);
     const int b = (int)blockIdx.x - ((int)gridDim.x - nbc); // boundary nodes first
-    if (b >= 0) sparse_node<ST, PH, PSTEP, ACCF>(a, b);
+    if (b >= 0) sparse_node<ST, PH, PSTEP, ACCF>(a, a.rev ? nbc - 1 - b : b);
     else special_node<ST, PH, PSTEP, ACCF>(a, (int)blockIdx.x);
 }
 

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_TMA) lbm_step_tma_kernel(c
     const int32_t Np = (int32_t)a.Np;
     int tile = blockIdx.x;
     int it = 0;
-    if (tile < ntiles && t == 0) tma_issue<S, PSTEP>(a, tile, buf0, &bar[0]);
+    if (tile < ntiles && t == 0) tma_issue<S, PSTEP>(a, a.rev ? ntiles - 1 - tile : tile, buf0, &bar[0]);
     // boundary nodes while the first tile arrives
     for (int sb = blockIdx.x; sb < nspecial_blocks; sb += gridDim.x) special_node<ST, PH, PSTEP, ACCF>(a, sb);
     for (; tile < ntiles; tile += gridDim.x, ++it) {
@@ -136,10 +136,11 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_TMA) lbm_step_tma_kernel(c
         const int next = tile + gridDim.x;
         if (next < ntiles && t == 0) {
             fence_proxy_async_smem();
-            tma_issue<S, PSTEP>(a, next, (it & 1) ? buf0 : buf1, &bar[(it + 1) & 1]);
+            tma_issue<S, PSTEP>(a, a.rev ? ntiles - 1 - next : next, (it & 1) ? buf0 : buf1, &bar[(it + 1) & 1]);
         }
-        const int row = tile / a.kblocks;
-        const int k0 = (tile - row * a.kblocks) * G::TW;
+        const int place = a.rev ? ntiles - 1 - tile : tile;
+        const int row = place / a.kblocks;
+        const int k0 = (place - row * a.kblocks) * G::TW;
         const int k = k0 + t;
         const int32_t n = row * a.nz + k;
         uint8_t cls = CLS_SOLID;
@@ -286,17 +287,18 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_H2) lbm_step_tma_h2_kernel
     const int32_t Np = (int32_t)a.Np;
     int tile = blockIdx.x;
     int it = 0;
-    if (tile < ntiles && t == 0) h2_issue(a, tile, kb2, buf0, &bar[0]);
+    if (tile < ntiles && t == 0) h2_issue(a, a.rev ? ntiles - 1 - tile : tile, kb2, buf0, &bar[0]);
     for (int sb = blockIdx.x; sb < nspecial_blocks; sb += gridDim.x) special_node<StoreF16, PH, false, ACCF>(a, sb);
     for (; tile < ntiles; tile += gridDim.x, ++it) {
         const __half *cur = (it & 1) ? buf1 : buf0;
         const int next = tile + gridDim.x;
         if (next < ntiles && t == 0) {
             fence_proxy_async_smem();
-            h2_issue(a, next, kb2, (it & 1) ? buf0 : buf1, &bar[(it + 1) & 1]);
+            h2_issue(a, a.rev ? ntiles - 1 - next : next, kb2, (it & 1) ? buf0 : buf1, &bar[(it + 1) & 1]);
         }
-        const int row = tile / kb2;
-        const int kA = (tile - row * kb2) * G::TW + 2 * t;
+        const int place = a.rev ? ntiles - 1 - tile : tile;
+        const int row = place / kb2;
+        const int kA = (place - row * kb2) * G::TW + 2 * t;
         const int32_t nA = row * a.nz + kA;
         // class bytes of both sites in one 16-bit load (nA is even)
         const uint32_t cl = __ldg((const unsigned short *)(a.ncls + nA));
