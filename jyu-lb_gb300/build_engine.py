@@ -24,8 +24,8 @@ COMMON = ["-std=c++20", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 HOST_FLAGS = ["-x", "cu", "-Xcompiler", "-fopenmp", "-Xcompiler", "-ffp-contract=off"]
 UNITS = {
     # 4 resident blocks (128 registers): the FP64 pipe and the integer pipes
-    # work for different warps at once.  128^3 TRT cavity 671 / 591 / 559 /
-    # 570 us a step at 2 / 3 / 4 / 5
+    # work for different warps at once.  At 3 / 4 / 5 blocks, us a step: 128^3
+    # TRT cavity 463 / 452 / 444, 4x34x4 channel 7.3 / 7.9 / 8.5
     "lbm_fp64.cu": ["-fmad=false", "-DJLB_MIN_BLOCKS=4"],
     # the fast FP64 step: contracted on purpose.  5 resident blocks (96
     # registers, a few spilled): 256^3 TRT cavity 1390 / 1197 / 1178 us a step

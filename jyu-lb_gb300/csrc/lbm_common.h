@@ -107,8 +107,8 @@ struct Consts64 {
     double c2;         // 1 - we/2
     double c3, c4, r9; // 1 - (we + wo)/2, (we - wo)/2, 1 - we
     // the same for the integer product (soft64::mul), with the projection's
-    // 1/72 and 1/36; `nonzero` has a bit for each of c3, c4, r9 that is not 0
-    soft64::MulC mc3, mc4, mr9, m72, m36;
+    // 1/72 and 1/36 and its factors 3, 6 and 18; `nonzero` has a bit for each of c3, c4, r9 that is not 0
+    soft64::MulC mc3, mc4, mr9, m72, m36, mwe, mwo, m3, m6, m18;
     unsigned nonzero;
     int soft; // 1: every constant is zero or well inside the normal range
 };
@@ -185,11 +185,18 @@ inline void set_consts64(StepArgs &a, int scheme) {
     k.r9 = 1.0 - a.w_e;
     k.m72 = soft64::make_mulc(1.0 / 72.0);
     k.m36 = soft64::make_mulc(2.0 * (1.0 / 72.0));
+    k.m3 = soft64::make_mulc(3.0);
+    k.m6 = soft64::make_mulc(6.0);
+    k.m18 = soft64::make_mulc(18.0);
+    k.mwe = soft64::make_mulc(k.we);
+    k.mwo = soft64::make_mulc(k.wodd);
     k.mc3 = soft64::make_mulc(k.c3);
     k.mc4 = soft64::make_mulc(k.c4);
     k.mr9 = soft64::make_mulc(k.r9);
     k.nonzero = 0;
-    k.soft = 1;
+    k.soft = k.we > 0x1p-100 && k.we < 2.0 && k.wodd > 0x1p-100 && k.wodd < 2.0;
+    for (int d = 0; d < 3; ++d) // a force too small for sums of normal numbers
+        if (a.g[d] != 0.0 && !(std::fabs(a.g[d]) > 0x1p-300 && std::fabs(a.g[d]) < 1.0)) k.soft = 0;
     const double rel[3] = {k.c3, k.c4, k.r9};
     for (int i = 0; i < 3; ++i) {
         if (rel[i] != 0.0) k.nonzero |= 1u << i;

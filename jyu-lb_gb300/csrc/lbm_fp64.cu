@@ -19,12 +19,15 @@ namespace jlb {
 //   * constants of the rates and the uniform force come from the host
 //     (StepArgs::k64, the same IEEE operations), not from every thread;
 //   * terms of force components that are zero add zeros, and are left out;
-//   * the bulk of the sites (collide_int) does the additions of the moments
-//     and the products with constants on the integer pipes, beside the FP64
-//     pipe.
-// Same bits as the plain form.  128^3 cavity, us a step (plain, fewer FP64
-// operations, with the integer form): TRT 1111, ~925, 559; BGK 938, -, 487;
-// regularized 938, -, 518.  Duct 100x61x47 TRT 161, 133, 89.
+//   * the bulk of the sites (collide_int) does the additions of the moments,
+//     the reciprocal of the density, the products with constants and the sums
+//     and differences of the projection's even and odd parts on the integer
+//     pipes, beside the FP64 pipe: of about 210 FP64 operations of a TRT site
+//     77 are left, and both kinds of pipe take about as long.
+// Same bits as the plain form.  128^3 cavity, us a step: plain; with integer
+// moments and relaxation; with the reciprocal too; with the moments' and the
+// projection's constants; with its sums: TRT 1111, 562, 548, 490, 452; BGK 938,
+// 497, 479, 425, 383; regularized 938, 521, 502, 402, 366.
 template <int SCH> struct Phys64 : Phys64Base {
     static constexpr bool host_consts = true;
 
@@ -72,21 +75,30 @@ template <int SCH> struct Phys64 : Phys64Base {
         put(9, __fma_rn(-0.5, h[4] + h[7] + h[9], (1.0 / 3.0) * h[0]));
     }
 
+    // products with the positive constants of the rates and the projection:
+    // integer ones in the integer form
+    template <bool INT> __device__ static C times(C x, C k, const soft64::MulC &m) {
+        if constexpr (INT) return soft64::mulz(x, m);
+        else return x * k;
+    }
     // relaxed moments of BGK / TRT from den and the stored velocity
-    __device__ static void relaxed_moments(C *h, const Force64 &F, const Consts64 &k, C den, C &ux, C &uy, C &uz) {
+    template <bool INT> __device__ static void relaxed_moments(C *h, const Force64 &F, const Consts64 &k, C den, C &ux, C &uy, C &uz) {
         if (F.mask & 1u) ux = __fma_rn(0.5, F.a[0], ux);
         if (F.mask & 2u) uy = __fma_rn(0.5, F.a[1], uy);
         if (F.mask & 4u) uz = __fma_rn(0.5, F.a[2], uz);
         const C jx = den * ux, jy = den * uy, jz = den * uz;
-        h[0] = den * k.we; h[1] = jx * k.wodd; h[2] = jy * k.wodd; h[3] = jz * k.wodd;
-        h[4] = jx * ux * k.we; h[5] = jx * uy * k.we; h[6] = jx * uz * k.we;
-        h[7] = jy * uy * k.we; h[8] = jy * uz * k.we; h[9] = jz * uz * k.we;
+        h[0] = times<INT>(den, k.we, k.mwe);
+        h[1] = times<INT>(jx, k.wodd, k.mwo); h[2] = times<INT>(jy, k.wodd, k.mwo); h[3] = times<INT>(jz, k.wodd, k.mwo);
+        h[4] = times<INT>(jx * ux, k.we, k.mwe); h[5] = times<INT>(jx * uy, k.we, k.mwe);
+        h[6] = times<INT>(jx * uz, k.we, k.mwe); h[7] = times<INT>(jy * uy, k.we, k.mwe);
+        h[8] = times<INT>(jy * uz, k.we, k.mwe); h[9] = times<INT>(jz * uz, k.we, k.mwe);
         force(h, F, k, den, jx, jy, jz);
     }
     // regularized: h holds the moments of f; relaxes them and sets the
     // stored velocity
-    __device__ static void relaxed_moments_reg(C *h, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz) {
-        const C den = h[0], inv = 1.0 / den;
+    template <bool INT>
+    __device__ static void relaxed_moments_reg(C *h, const Force64 &F, const Consts64 &k, C inv, C &ux, C &uy, C &uz) {
+        const C den = h[0];
         C jx = h[1], jy = h[2], jz = h[3];
         if (F.mask & 1u) jx = __fma_rn(0.5, F.a[0] * den, jx);
         if (F.mask & 2u) jy = __fma_rn(0.5, F.a[1] * den, jy);
@@ -95,7 +107,11 @@ template <int SCH> struct Phys64 : Phys64Base {
         const C ex = den * ux, ey = den * uy, ez = den * uz;
         const C he[10] = {den, ex, ey, ez, ex * ux, ex * uy, ex * uz, ey * uy, ey * uz, ez * uz};
 #pragma unroll
-        for (int m = 0; m < 10; ++m) h[m] = h[m] * k.r9 + k.we * he[m];
+        for (int m = 0; m < 10; ++m) {
+            const C e = times<INT>(he[m], k.we, k.mwe);
+            if (INT && !(k.nonzero & 4u)) h[m] = e; // 1 - we = 0
+            else h[m] = times<INT>(h[m], k.r9, k.mr9) + e;
+        }
         force(h, F, k, den, jx, jy, jz);
     }
 
@@ -105,7 +121,7 @@ template <int SCH> struct Phys64 : Phys64Base {
         C h[10];
         if (SCH != SCH_REG) {
             const C den = f_to_den_vel(f, ux, uy, uz);
-            relaxed_moments(h, F, k, den, ux, uy, uz);
+            relaxed_moments<false>(h, F, k, den, ux, uy, uz);
             if (SCH == SCH_BGK) {
 #pragma unroll
                 for (int q = 0; q < Q; ++q) f[q] = f[q] * k.r9;
@@ -139,7 +155,7 @@ template <int SCH> struct Phys64 : Phys64Base {
             h[7] = (d1y + dy1) - d3;
             h[8] = f[5] + f[13] - f[7] - f[11];
             h[9] = (d1z + dz1) - d3;
-            relaxed_moments_reg(h, F, k, ux, uy, uz);
+            relaxed_moments_reg<false>(h, F, k, 1.0 / h[0], ux, uy, uz);
             project_fused<false>(h, f);
             return den;
         }
@@ -149,13 +165,14 @@ template <int SCH> struct Phys64 : Phys64Base {
         return collide(f, F, k, u[0], u[1], u[2]);
     }
 
-    // The same update, with the additions of the moments and the products with
-    // constants on the integer pipes (soft64.cuh): the same bits.  It needs
-    // populations in [2^-9, 1/4) (rest: up to 1/2) and projections that are
-    // positive; anything else sets `bad` and leaves f undefined.
+    // The same update, with most of its operations on the integer pipes
+    // (soft64.cuh): the same bits.  It needs populations in [2^-9, 1/4) (rest:
+    // up to 1/2), velocities that are zero or no smaller than 2^-400, and
+    // projections whose even parts outweigh the odd ones; anything else sets
+    // `bad` and leaves f undefined.
     __device__ static C collide_int(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz, bool &bad) {
         using namespace soft64;
-        C h[10], den;
+        C h[10], den, inv;
         uint32_t range = 0, range9 = 0, least = 0;
         {
             uint64_t x[Q];
@@ -166,7 +183,9 @@ template <int SCH> struct Phys64 : Phys64Base {
             const uint64_t d01y = add(add(x[5], x[6]), x[7]);
             const uint64_t d0y1 = add(add(x[11], x[12]), x[13]);
             const uint64_t xx = add(d1x, dx1);
-            den = to_double(add(add(add(add(add(xx, d01y), d0y1), x[8]), x[9]), x[10]));
+            const uint64_t xd = add(add(add(add(add(xx, d01y), d0y1), x[8]), x[9]), x[10]);
+            den = to_double(xd);
+            inv = recip(xd);
             const C jx = diff_to_double(dx1, d1x);
             if (SCH != SCH_REG) {
                 // jyulb/D3Q19.pyx:348-390
@@ -174,7 +193,6 @@ template <int SCH> struct Phys64 : Phys64Base {
                 const uint64_t zp = add(add(add(add(x[3], x[7]), x[10]), x[13]), x[17]);
                 const uint64_t z = sub(sub(sub(sub(zp, x[1], least), x[5], least), x[8], least), x[11], least);
                 const C jy = diff_to_double(y, x[14]), jz = diff_to_double(z, x[15]);
-                const C inv = 1.0 / den;
                 ux = inv * jx; uy = inv * jy; uz = inv * jz;
             } else {
                 // jyulb/D3Q19.pyx:395-452
@@ -192,7 +210,7 @@ template <int SCH> struct Phys64 : Phys64Base {
             }
         }
         if (SCH != SCH_REG) {
-            relaxed_moments(h, F, k, den, ux, uy, uz);
+            relaxed_moments<true>(h, F, k, den, ux, uy, uz);
             if (SCH == SCH_BGK) {
                 // 1 - we = 0 (tau = 1) leaves the projection alone
                 if (k.nonzero & 4u) {
@@ -230,43 +248,51 @@ template <int SCH> struct Phys64 : Phys64Base {
                 f[9] = k.nonzero & 4u ? mul(f[9], k.mr9) : 0.0;
             }
         } else {
-            relaxed_moments_reg(h, F, k, ux, uy, uz);
+            relaxed_moments_reg<true>(h, F, k, inv, ux, uy, uz);
         }
         uint32_t span = 0;
-        project_int<SCH != SCH_REG>(h, k, f, span);
-        bad = range > 6u || range9 > 7u || least >= (1u << 31) - (1u << 21) || span > PROJ_SPAN;
+        int32_t apart = 1 << 30;
+        project_int<SCH != SCH_REG>(h, k, f, span, apart);
+        // velocities are zero or at least 2^-400: their products are normal
+        uint32_t tiny = 0xffffffffu;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const uint64_t u = bits(d == 0 ? ux : d == 1 ? uy : uz);
+            const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+            const uint32_t z = (u << 1) ? e : 0x7ffu;
+            tiny = tiny < z ? tiny : z;
+        }
+        bad = range > 6u || range9 > 7u || least >= (1u << 31) - (1u << 21) || span > PROJ_SPAN || apart < 2 ||
+              tiny < 1023u - 400u;
         return den;
     }
 
-    // project_fused with integer products; `span` exceeds PROJ_SPAN unless
-    // every projection argument lies in [2^-40, 2^10)
+    // project_fused with integer products and sums; `span` exceeds PROJ_SPAN
+    // unless every even part lies in [2^-40, 2^10), and `apart` is below 2 where
+    // an odd part is not below a quarter of its even one
     static constexpr uint32_t PROJ_LO = (1023u - 40u) << 20, PROJ_SPAN = (50u << 20) - 1u;
-    template <bool ADD> __device__ static void project_int(const C *h, const Consts64 &k, C *f, uint32_t &span) {
-        const C t4 = 3.0 * h[4], t7 = 3.0 * h[7], t9 = 3.0 * h[9];
+    template <bool ADD>
+    __device__ static void project_int(const C *h, const Consts64 &k, C *f, uint32_t &span, int32_t &apart) {
+        const C t4 = soft64::mulz(h[4], k.m3), t7 = soft64::mulz(h[7], k.m3), t9 = soft64::mulz(h[9], k.m3);
         const C s = h[0] + t4, v = __fma_rn(2.0, h[0], -t4);
         const C w = __fma_rn(2.0, s, -t7), v2 = __fma_rn(2.0, t7, v);
         const C exy = __fma_rn(2.0, s + t7, -t9), exz = __fma_rn(2.0, t9, w), eyz = __fma_rn(2.0, t9, v2);
         const C ex = w - t9, ey = v2 - t9, ez = __fma_rn(2.0, t9, v - t7);
-        const C q1 = 6.0 * h[1], q2 = 6.0 * h[2], q3 = 6.0 * h[3];
-        auto scaled = [&](C y, const soft64::MulC &m) {
-            const uint32_t e = (uint32_t)__double2hiint(y) - PROJ_LO;
-            span = span > e ? span : e;
-            return soft64::mul(y, m);
-        };
+        const C q1 = soft64::mulz(h[1], k.m6), q2 = soft64::mulz(h[2], k.m6), q3 = soft64::mulz(h[3], k.m6);
         auto put = [&](int q, C p) { f[q] = ADD ? f[q] + p : p; };
-        auto pair = [&](int lo, C e, C o) {
-            put(lo, scaled(e - o, k.m72));
-            put(18 - lo, scaled(e + o, k.m72));
-        };
-        auto axis = [&](int lo, C e, C o) {
-            put(lo, scaled(e - o, k.m36));
-            put(18 - lo, scaled(e + o, k.m36));
+        auto both = [&](int lo, C e, C o, const soft64::MulC &m) { // f_lo from e - o, its opposite from e + o
+            const uint32_t x = (uint32_t)__double2hiint(e) - PROJ_LO;
+            span = span > x ? span : x;
+            C plus, minus;
+            soft64::add_sub(e, o, plus, minus, apart);
+            put(lo, soft64::mul(minus, m));
+            put(18 - lo, soft64::mul(plus, m));
         };
         C o;
-        o = 18.0 * h[5]; pair(0, exy + o, q1 + q2); pair(4, exy - o, q1 - q2);
-        o = 18.0 * h[6]; pair(1, exz + o, q1 + q3); pair(3, exz - o, q1 - q3);
-        o = 18.0 * h[8]; pair(5, eyz + o, q2 + q3); pair(7, eyz - o, q2 - q3);
-        axis(2, ex, q1); axis(6, ey, q2); axis(8, ez, q3);
+        o = soft64::mulz(h[5], k.m18); both(0, exy + o, q1 + q2, k.m72); both(4, exy - o, q1 - q2, k.m72);
+        o = soft64::mulz(h[6], k.m18); both(1, exz + o, q1 + q3, k.m72); both(3, exz - o, q1 - q3, k.m72);
+        o = soft64::mulz(h[8], k.m18); both(5, eyz + o, q2 + q3, k.m72); both(7, eyz - o, q2 - q3, k.m72);
+        both(2, ex, q1, k.m36); both(6, ey, q2, k.m36); both(8, ez, q3, k.m36);
         put(9, __fma_rn(-0.5, h[4] + h[7] + h[9], (1.0 / 3.0) * h[0]));
     }
 };

@@ -116,6 +116,43 @@ S64_FN double mul(double x, const MulC &k) {
     return from((uint32_t)(m >> 32) + (xh & 0xfff00000u) + k.base + (c << 20), (uint32_t)m);
 }
 
+// x * k for k > 0 where x may also be a zero (the product is then that zero);
+// not for denormal x
+S64_FN double mulz(double x, const MulC &k) {
+    const double p = mul(x, k);
+    const uint32_t xh = (uint32_t)(bits(x) >> 32);
+    const bool zero = (xh & 0x7ff00000u) == 0u;
+    return zero ? from(xh & 0x80000000u, 0u) : p;
+}
+
+// e + o and e - o for normal e > 0 and |o| < e / 4 (o zero or normal): o is
+// aligned to e's last place with 9 more bits and a sticky one, added and
+// subtracted, and both results rounded.  `least` collects the exponent
+// difference, below 2 for a larger o.
+S64_FN void add_sub(double e, double o, double &plus, double &minus, int32_t &least) {
+    const uint64_t ue = bits(e), uo = bits(o);
+    const uint32_t eh = (uint32_t)(ue >> 32), oh = (uint32_t)(uo >> 32);
+    const uint32_t oe = (oh >> 20) & 0x7ffu;
+    const int32_t r = (int32_t)(eh >> 20) - (int32_t)oe;
+    least = least < r ? least : r;
+    const uint64_t me = ((ue & 0xfffffffffffffull) | (1ull << 52)) << 9;
+    const uint64_t mo = ((uo & 0xfffffffffffffull) | ((uint64_t)(oe < 1u ? oe : 1u) << 52)) << 9;
+    const uint32_t sh = (uint32_t)r & 0x80000000u ? 0u : (uint32_t)r < 63u ? (uint32_t)r : 63u;
+    const uint64_t v = mo >> sh;
+    const uint64_t jam = v | ((v << sh) != mo ? 1u : 0u);
+    auto round = [&](uint64_t s) { // [3/4 2^61, 5/4 2^62)
+        const uint32_t hi = (uint32_t)(s >> 32), lo = (uint32_t)s;
+        const uint32_t d = (top_bit(hi) - 20u) & 31u;
+        const uint32_t mask = low_mask(d), odd = (lo >> d) & 1u;
+        s += (mask >> 1) + odd;
+        return from(((uint32_t)(s >> 32) >> d) + ((eh & 0xfff00000u) + ((d - 10u) << 20)), shr_lo((uint32_t)s, (uint32_t)(s >> 32), d));
+    };
+    const double sum = round(me + jam), dif = round(me - jam);
+    const bool neg = (oh >> 31) != 0u;
+    plus = neg ? dif : sum;
+    minus = neg ? sum : dif;
+}
+
 // ---------------------------------------------------------------------------
 // Chains of additions in fixed point with unit 2^-61.  Each add() rounds as
 // the FP64 addition does: to 53 significant bits of the partial sum.
@@ -157,6 +194,42 @@ S64_FN double to_double(uint64_t s) {
     const uint32_t hi = (uint32_t)(s >> 32), lo = (uint32_t)s;
     const uint32_t d = top_bit(hi) - 20u;
     return from((hi >> d) + ((d + FIX_E0 - 1u) << 20), shr_lo(lo, hi, d));
+}
+// 1 / s for a fixed-point number rounded to 53 bits, as the correctly rounded
+// double.  With s = D 2^d, D of 53 bits, it is q 2^(-44 - d) for the integer q
+// nearest 2^105 / D: two Newton steps (x <- x + x (1 - D x)) from a 23-bit
+// reciprocal give q to within one, and the remainder 2^105 - D q, below 2^54
+// in size and so known from its low 64 bits, decides.  (No quotient lies
+// midway: 2^106 / D would be an odd integer.)
+S64_FN double recip(uint64_t s) {
+    const uint32_t d = (top_bit((uint32_t)(s >> 32)) - 20u) & 31u;
+    const uint64_t D = s >> d, dn = D << 11; // dn / 2^64 in [1/2, 1)
+    const uint32_t dh = (uint32_t)(dn >> 32);
+    // x0 / 2^30 = 2^64 / dn to about 2^-22, from the leading 24 bits
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3f000000u | ((dh >> 8) & 0x7fffffu))));
+    const uint32_t x0 = (uint32_t)(y * 1073741824.0f);
+#else
+    const uint32_t x0 = (uint32_t)((1.0f / ((float)(dh >> 8) * 5.9604644775390625e-8f)) * 1073741824.0f);
+#endif
+    // e / 2^62 = 1 - dn x0 / 2^94, |e| < 2^42
+    const uint64_t t = (uint64_t)dh * x0 + (((uint64_t)(uint32_t)dn * x0) >> 32);
+    const int64_t e = (int64_t)((1ull << 62) - t);
+    // x1 / 2^62, to about 2^-43
+    const int64_t x1 = ((int64_t)x0 << 32) + (((e >> 12) * (int64_t)x0) >> 18);
+    // the second step: e1 / 2^62 = 1 - dn x1 / 2^126, |e1| < 2^20
+    const uint64_t xl = (uint32_t)x1, xh = (uint64_t)x1 >> 32;
+    const uint64_t m1 = (uint64_t)dh * xl + (((uint64_t)(uint32_t)dn * xl) >> 32);
+    const uint64_t m2 = (uint64_t)(uint32_t)dn * xh + (uint32_t)m1;
+    const uint64_t p = (uint64_t)dh * xh + (m1 >> 32) + (m2 >> 32);
+    const int64_t e1 = (int64_t)((1ull << 62) - p);
+    const int64_t x2 = x1 + ((e1 * (int64_t)(x1 >> 32)) >> 30);
+    uint64_t q = (uint64_t)(x2 + 512) >> 10; // x2 / 2^62 = 2^53 / D
+    const int64_t rem = -(int64_t)(D * q);  // 2^105 - D q
+    q += 2 * rem > (int64_t)D;
+    q -= 2 * rem < -(int64_t)D;
+    return from((uint32_t)(q >> 32) + ((1030u - d) << 20), (uint32_t)q);
 }
 // the signed difference a - b (|a - b| < 2^63 units) rounded to a double; an
 // exact zero is +0 as in IEEE subtraction

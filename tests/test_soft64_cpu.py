@@ -18,6 +18,22 @@ extern "C" {
 void s_mul(const double *x, const double *k, double *o, long n) {
     for (long i = 0; i < n; ++i) o[i] = mul(x[i], make_mulc(k[i]));
 }
+void s_mulz(const double *x, const double *k, double *o, long n) {
+    for (long i = 0; i < n; ++i) o[i] = mulz(x[i], make_mulc(k[i]));
+}
+void s_recip(const double *x, double *o, long n) {
+    for (long i = 0; i < n; ++i) {
+        uint32_t range = 0;
+        o[i] = recip(fix(x[i], range));
+    }
+}
+void s_add_sub(const double *e, const double *o, double *p, double *m, int *least, long n) {
+    for (long i = 0; i < n; ++i) {
+        int32_t l = 1 << 30;
+        add_sub(e[i], o[i], p[i], m[i], l);
+        least[i] = l;
+    }
+}
 // o0 = (x + y) + z, o1 = (x + y) - z, o2 = x - y; r, p as the callers check them
 void s_chain(const double *x, const double *y, const double *z, double *o0, double *o1, double *o2,
              unsigned *r, unsigned *p, long n) {
@@ -107,3 +123,36 @@ def test_range_check_sees_other_numbers(lib, bad):
     r, p = np.empty(1, np.uint32), np.empty(1, np.uint32)
     lib.s_chain(ptr(x), ptr(y), ptr(z), *(ptr(v) for v in o), ptr(r), ptr(p), ctypes.c_long(1))
     assert r[0] > 7
+
+
+def test_product_of_zeros(lib):
+    x = np.array([0.0, -0.0, 1.5, -1.5] * 3)
+    k = np.repeat([3.0, 18.0, 1 / 72], 4)
+    o = np.empty(12)
+    lib.s_mulz(ptr(x), ptr(k), ptr(o), ctypes.c_long(12))
+    assert same_bits(o, x * k)
+
+
+def test_reciprocals(lib):
+    rng = np.random.default_rng(7)
+    n = 2_000_000
+    x = numbers(rng, n, -8, 1)
+    # the ends of a binade, where the quotient's own binade changes
+    x[:6] = [1.0, 0.5, 2.0, np.nextafter(1, 2), np.nextafter(1, 0), np.nextafter(2, 1)]
+    o = np.empty(n)
+    lib.s_recip(ptr(x), ptr(o), ctypes.c_long(n))
+    assert same_bits(o, 1.0 / x)
+
+
+def test_sums_and_differences(lib):
+    rng = np.random.default_rng(8)
+    n = 2_000_000
+    e = numbers(rng, n, -40, 9)
+    o = np.ldexp(numbers(rng, n, 0, 0, True), np.frexp(e)[1] - 1 - rng.integers(0, 75, n))
+    o[: n // 50] = 0.0
+    o[n // 50: n // 25] = -0.0
+    p, m, least = np.empty(n), np.empty(n), np.empty(n, np.int32)
+    lib.s_add_sub(ptr(e), ptr(o), ptr(p), ptr(m), ptr(least), ctypes.c_long(n))
+    fine = least >= 2
+    assert np.array_equal(fine, np.frexp(e)[1] - np.where(o == 0, -1023, np.frexp(o)[1]) >= 2)
+    assert same_bits(p[fine], (e + o)[fine]) and same_bits(m[fine], (e - o)[fine])
