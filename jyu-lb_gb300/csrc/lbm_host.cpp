@@ -1034,18 +1034,25 @@ int download(jlb_solver *s, double *den, double *vel) {
     return r;
 }
 
-// Halo rules of den / vel (enforce_den_vel) applied to the moments of the
-// last moment-writing step: the fluid sites of the layers they read are
-// written into the host arrays first (in place for page-locked arrays, else
-// by a full download)
-int halo_from_moments(jlb_solver *s, double *den, double *vel, unsigned axes) {
+// Halo rules of den / vel: by a kernel on page-locked arrays, else on the
+// host.  from_moments: on the moments of the last moment-writing step, whose
+// fluid sites need not have reached the host arrays
+int halo_rules(jlb_solver *s, double *den, double *vel, bool from_moments) {
     double *dd = (double *)dev_view(den), *dv = (double *)dev_view(vel);
     if (dd && dv) {
-        CKR(aux_download_layers(s->prec, s->geom, axes, s->nmask, s->mom[0], s->mom[1], s->mom[2], s->mom[3], dd, dv,
-                                s->st));
+        int rule[6];
+        bool any = false;
+        for (int f = 0; f < 6; ++f) {
+            const int b = s->cfg.bc[f];
+            rule[f] = b == BC_PERIODIC ? 1 : b == BC_SYMMETRIC ? 2 : 0;
+            any = any || rule[f];
+        }
+        if (!any) return JLB_OK;
+        CKR(aux_halo(s->prec, s->geom, rule, s->nmask, from_moments ? s->mom : nullptr, dd, dv, s->st));
         ++s->launches;
-        CK(cudaStreamSynchronize(s->st));
-    } else {
+        return JLB_OK;
+    }
+    if (from_moments) {
         int r = download(s, den, vel);
         if (r) return r;
     }
@@ -1420,7 +1427,7 @@ int jlb_evolve(jlb_solver *s, uint32_t tsteps, const double g[3], double *den, d
     using clk = std::chrono::steady_clock;
     auto since = [](clk::time_point a) { return std::chrono::duration<double>(clk::now() - a).count(); };
     const auto t_start = clk::now();
-    enforce_den_vel(s, den, vel);
+    if (int rh = halo_rules(s, den, vel, false)) return rh;
     // solid velocities: reclassify when any of them changed since the last call
     int changed = 0;
     const int64_t nchk = (int64_t)s->wall_chk.size();
@@ -1457,16 +1464,13 @@ int jlb_evolve(jlb_solver *s, uint32_t tsteps, const double g[3], double *den, d
     // The reference refreshes the periodic / symmetric halos of den and vel
     // at the start of every step (jyulb/isothermal.pyx:1408-1411), so after
     // evolve(n) they hold the images of step n-1's moments: run n-1 steps with
-    // moments, bring the layers the halo rules read into the host arrays,
-    // apply the rules, then the last step (whose download rewrites the fluid
-    // sites of those layers)
-    unsigned halo_axes = 0;
-    for (int face = 0; face < 6; ++face)
-        if (s->cfg.bc[face] == BC_PERIODIC || s->cfg.bc[face] == BC_SYMMETRIC) halo_axes |= 1u << (face >> 1);
+    // moments, apply the rules to those, then the last step
+    bool halo = false;
+    for (int face = 0; face < 6; ++face) halo = halo || s->cfg.bc[face] == BC_PERIODIC || s->cfg.bc[face] == BC_SYMMETRIC;
     uint32_t remaining = tsteps;
-    if (halo_axes && tsteps >= 2) {
+    if (halo && tsteps >= 2) {
         if ((r = run_steps(s, tsteps - 1, true))) return r;
-        if ((r = halo_from_moments(s, den, vel, halo_axes))) return r;
+        if ((r = halo_rules(s, den, vel, true))) return r;
         remaining = 1;
     }
     r = run_steps(s, overlap ? remaining - 1 : remaining, !overlap);
