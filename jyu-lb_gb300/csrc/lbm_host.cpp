@@ -970,12 +970,19 @@ cudaError_t copy_interior(const jlb_solver *s, const double *src, double *dst, i
 // The copy-engine download applies when every interior site is fluid (the
 // host values of solid sites must stay untouched, so they cannot be
 // overwritten by a box copy) and den/vel are page-locked; it needs a device
-// copy of the host layout (allocated on first use).  JLB_DMA_DOWNLOAD=0
-// keeps the kernel path.
+// copy of the host layout (allocated on first use).  It also wants enough
+// sites: its slabs cost some 40 enqueued operations, and its pitched copies of
+// short rows run below the kernel's stores, but it hides the copy behind the
+// step, the more the slower the step.  evolve(1) of a cavity, copy engine /
+// kernel, us: FP32 20x18x16 86 / 37, 60x57x56 124 / 92, 128x100x90 372 / 328,
+// 128^3 564 / 553, 192x128x128 794 / 815; FP64 20x18x16 139 / 50, 90x80x70 342 /
+// 278, 128x100x90 533 / 551, 128^3 786 / 938; fast FP64 128x100x90 401 / 388,
+// 128^3 584 / 648.  JLB_DMA_DOWNLOAD=0 keeps the kernel path, 1 the copies.
 bool dma_ready(jlb_solver *s, double *den, double *vel) {
     const char *de = std::getenv("JLB_DMA_DOWNLOAD");
-    const bool dma_off = de && de[0] == '0';
-    if (dma_off || s->stg_failed || s->nfluid != (uint64_t)s->N || !dev_view(den) || !dev_view(vel)) return false;
+    const int64_t least = s->prec == PREC_FP64 ? (int64_t)1 << 20 : (int64_t)5 << 19;
+    const bool off = de && de[0] ? de[0] == '0' : s->N < least;
+    if (off || s->stg_failed || s->nfluid != (uint64_t)s->N || !dev_view(den) || !dev_view(vel)) return false;
     if (!s->stg_den) {
         const size_t nb = (size_t)s->NCNT * sizeof(double);
         if (cudaMalloc(&s->stg_den, nb) != cudaSuccess || cudaMalloc(&s->stg_vel, 3 * nb) != cudaSuccess) {
