@@ -72,6 +72,7 @@ class Ensemble:
             raise (ValueError if rc == _native.JLB_ERR_INVALID_ARG else RuntimeError)(msg)
         self._h = h
         self.tot_tsteps = 0
+        self._solid = [np.flatnonzero(d.phase == 0) for d in self.domains]
 
     def __del__(self):
         h = getattr(self, '_h', None)
@@ -104,8 +105,10 @@ class Ensemble:
         domain's input values."""
         dom = self.domains[d]
         sh = dom.phase.shape
-        den = np.ones(sh) if dom.den is None else dom.den.copy()
-        vel = np.zeros(sh + (3,)) if dom.vel is None else dom.vel.copy()
+        # the engine writes every fluid site: only the solid ones need values
+        den, vel, solid = np.empty(sh), np.empty(sh + (3,)), self._solid[d]
+        den.reshape(-1)[solid] = 1.0 if dom.den is None else dom.den.reshape(-1)[solid]
+        vel.reshape(-1, 3)[solid] = 0.0 if dom.vel is None else dom.vel.reshape(-1, 3)[solid]
         self._check(self._lib.jlb_batch_moments(self._h, d, _native.dptr(den), _native.dptr(vel)))
         return den, vel
 
