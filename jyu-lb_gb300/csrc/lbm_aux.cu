@@ -565,6 +565,21 @@ int aux_sparse_tables(const int64_t *rd, const int64_t *wr, const int64_t *node,
     return (int)cudaGetLastError();
 }
 
+__global__ void sparse_classes_kernel(const uint8_t *ncls, const uint32_t *nmask, const int32_t *csite, int64_t Nc,
+                                      int64_t Npc, uint8_t *ccls, uint32_t *cmask) {
+    const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= Npc) return;
+    ccls[m] = m < Nc ? ncls[csite[m]] : CLS_SOLID;
+    cmask[m] = m < Nc ? nmask[csite[m]] : MASK_SOLID;
+}
+
+int aux_sparse_classes(const uint8_t *ncls, const uint32_t *nmask, const int32_t *csite, int64_t Nc, int64_t Npc,
+                       uint8_t *ccls, uint32_t *cmask, cudaStream_t st) {
+    if (Npc <= 0) return 0;
+    sparse_classes_kernel<<<nblk(Npc, 256), 256, 0, st>>>(ncls, nmask, csite, Nc, Npc, ccls, cmask);
+    return (int)cudaGetLastError();
+}
+
 int aux_download_rows(int prec, const AuxGeom &g, const uint32_t *nmask, const void *den, const void *ux,
                       const void *uy, const void *uz, double *hden, double *hvel, int64_t row0, int64_t nrows,
                       cudaStream_t st) {

@@ -29,6 +29,9 @@ int aux_sparse_pack(int elem_bytes, void *dense, void *comp, const int32_t *csit
 // boundary-node element tables (q * Np + n) -> fluid-only (q * Npc + m)
 int aux_sparse_tables(const int64_t *rd, const int64_t *wr, const int64_t *node, int M, const int32_t *cidx,
                       int64_t Np, int64_t Npc, int64_t *rdc, int64_t *wrc, int64_t *nodec, cudaStream_t st);
+// classes and masks of the fluid sites in their own order
+int aux_sparse_classes(const uint8_t *ncls, const uint32_t *nmask, const int32_t *csite, int64_t Nc, int64_t Npc,
+                       uint8_t *ccls, uint32_t *cmask, cudaStream_t st);
 // *flag = 1 (device-accessible int) when vel (device-accessible halo-padded
 // host array) differs from known (3 per position) at any of the nwall
 // positions

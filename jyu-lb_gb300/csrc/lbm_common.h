@@ -153,6 +153,8 @@ struct StepArgs {
     // fluid-only ("sparse") population layout, used on lattices with many
     // solid sites: populations f[q * Npc + m] over the fluid sites m only
     const int32_t *csite; // [Nc] lattice site n of fluid site m
+    const uint8_t *ccls;  // [Npc] node classes of the fluid sites (padding: CLS_SOLID)
+    const uint32_t *cmask; // [Npc] their node masks
     const int32_t *cidx;  // [N] fluid index m of lattice site n (-1: solid)
     int64_t Nc, Npc;      // fluid sites, their slot stride (multiple of 128)
     float inv_syz, inv_nz; // 1/(ny*nz), 1/nz for the site -> (i,j,k) split; 0: use integer division

@@ -641,6 +641,8 @@ StepArgs make_args(const jlb_solver *s, int write_moments) {
         a.f = s->fc;
         a.csite = s->d_csite;
         a.cidx = s->d_cidx;
+        a.ccls = s->d_ccls;
+        a.cmask = s->d_cmask;
         a.Nc = s->Nc;
         a.Npc = s->Npc;
         // float-reciprocal split when every quotient (i < nx, j < ny) stays
@@ -811,10 +813,12 @@ int sparse_setup(jlb_solver *s) {
     s->Npc = ((s->Nc + 127) / 128) * 128;
     if (cudaMalloc(&s->fc, (size_t)19 * s->Npc * s->ssz) != cudaSuccess ||
         cudaMalloc(&s->d_csite, std::max<size_t>(1, csite.size()) * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&s->d_cidx, (size_t)s->N * sizeof(int32_t)) != cudaSuccess) {
+        cudaMalloc(&s->d_cidx, (size_t)s->N * sizeof(int32_t)) != cudaSuccess ||
+        cudaMalloc(&s->d_ccls, std::max<size_t>(1, (size_t)s->Npc)) != cudaSuccess ||
+        cudaMalloc(&s->d_cmask, std::max<size_t>(1, (size_t)s->Npc) * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(s->fc); cudaFree(s->d_csite); cudaFree(s->d_cidx);
-        s->fc = nullptr; s->d_csite = s->d_cidx = nullptr;
+        cudaFree(s->fc); cudaFree(s->d_csite); cudaFree(s->d_cidx); cudaFree(s->d_ccls); cudaFree(s->d_cmask);
+        s->fc = nullptr; s->d_csite = s->d_cidx = nullptr; s->d_ccls = nullptr; s->d_cmask = nullptr;
         s->sparse = false;  // not enough device memory: lattice layout
         ++s->args_version;
         return JLB_OK;
@@ -844,6 +848,10 @@ int sparse_enter(jlb_solver *s) {
         }
         CKR(aux_sparse_tables(s->d_sp_rd, s->d_sp_wr, s->d_sp_node, s->M, s->d_cidx, s->Np, s->Npc, s->d_sp_rd_c,
                               s->d_sp_wr_c, s->d_sp_cnode, s->st));
+        ++s->launches;
+    }
+    if (s->sp_tables_dirty) {
+        CKR(aux_sparse_classes(s->ncls, s->nmask, s->d_csite, s->Nc, s->Npc, s->d_ccls, s->d_cmask, s->st));
         ++s->launches;
     }
     s->sp_tables_dirty = false;
@@ -1287,7 +1295,7 @@ void jlb_destroy(jlb_solver *s) {
     void *bufs[] = {s->f, s->nmask, s->ncls, s->mom[0], s->mom[1], s->mom[2], s->mom[3], s->acc, s->red_partial,
                     s->red_out, s->d_sp_node, s->d_sp_info, s->d_sp_rd, s->d_sp_wr, s->d_sp_lw, s->d_sp_bc,
                     s->d_sp_den, s->d_err, s->fi_partial, s->fi_out, s->stg_den, s->stg_vel,
-                    s->fc, s->d_csite, s->d_cidx, s->d_sp_rd_c, s->d_sp_wr_c, s->d_sp_cnode,
+                    s->fc, s->d_csite, s->d_cidx, s->d_ccls, s->d_cmask, s->d_sp_rd_c, s->d_sp_wr_c, s->d_sp_cnode,
                     s->d_wall_pos, s->d_wall_vel, s->res_prev};
     for (void *p : bufs)
         if (p) cudaFree(p);

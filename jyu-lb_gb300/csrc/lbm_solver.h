@@ -48,6 +48,8 @@ struct jlb_solver {
     bool sp_tables_dirty = true;         // boundary tables changed since their translation
     void *fc = nullptr;                  // [19][Npc] populations of the fluid sites
     int32_t *d_csite = nullptr, *d_cidx = nullptr;
+    uint8_t *d_ccls = nullptr;           // [Npc] node classes of the fluid sites (padding: solid)
+    uint32_t *d_cmask = nullptr;         // [Npc] their node masks
     int64_t *d_sp_rd_c = nullptr, *d_sp_wr_c = nullptr, *d_sp_cnode = nullptr;
     int sp_c_cap = 0;
     int64_t Nc = 0, Npc = 0;
