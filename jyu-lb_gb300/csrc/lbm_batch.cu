@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(BLOCK, JLB_BATCH_WARPS * 32 / BLOCK)
     // itself is indexed by a 32-bit site
     const uint32_t m = (PSTEP && cls != BCLS_PLAIN) ? __ldg(a.nmask + n) : 0u;
     const uint32_t mv = (cls == BCLS_MOVING) ? __ldg(a.mmask + n) : 0u;
+    wait_previous();
     C fv[Q];
     int32_t dI[3], dJ[3], dK[3];
     if (PSTEP) {
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(BLOCK, JLB_BATCH_WARPS * 32 / BLOCK)
         }
         fv[q] = ST::template ld<q>(p);
     });
+    let_next_start();
     if (mv) {
         // Ladd's term on links to moving solids: 6 w_q rho_prev (c_q . U)
         const float dprev = a.dprev[n];
@@ -148,9 +150,10 @@ __global__ void __launch_bounds__(BLOCK, JLB_BATCH_WARPS * 32 / BLOCK)
 
 int launch_batch_step(const BatchArgs &a, int scheme, bool pstep, int block, int ntiles, cudaStream_t st) {
     const bool idx32 = 19 * a.Np < (int64_t(1) << 32);
+    cudaError_t r = cudaSuccess;
 #define JLB_B(SCH, P, B)                                                                 \
-    if (idx32) lbm_batch_kernel<SCH, P, B, true><<<ntiles, B, 0, st>>>(a);               \
-    else lbm_batch_kernel<SCH, P, B, false><<<ntiles, B, 0, st>>>(a)
+    if (idx32) r = launch_step(lbm_batch_kernel<SCH, P, B, true>, dim3(ntiles), dim3(B), 0, st, a);  \
+    else r = launch_step(lbm_batch_kernel<SCH, P, B, false>, dim3(ntiles), dim3(B), 0, st, a)
 #define JLB_BB(SCH, B) if (pstep) JLB_B(SCH, true, B); else JLB_B(SCH, false, B);
 #define JLB_BS(SCH)                               \
     if (block == 64) { JLB_BB(SCH, 64) }          \
@@ -162,7 +165,8 @@ int launch_batch_step(const BatchArgs &a, int scheme, bool pstep, int block, int
 #undef JLB_BS
 #undef JLB_BB
 #undef JLB_B
-    return (int)cudaGetLastError();
+    const cudaError_t l = cudaGetLastError();
+    return (int)(r != cudaSuccess ? r : l);
 }
 
 // Boundary nodes: the single-domain boundary-node step with the relaxation

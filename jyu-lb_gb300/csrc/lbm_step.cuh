@@ -198,6 +198,40 @@ __device__ __forceinline__ int32_t split_div(int32_t l, int32_t d, float inv, in
     return q;
 }
 
+// Programmatic dependent launch between the steps of a stream or graph: a
+// step's blocks may become resident while the step before drains, work out
+// their sites and read the static classes, and wait here, before any
+// population, for that step to be complete and its stores visible.  Every
+// fluid site's thread waits, so a step cannot complete before the one before
+// it, however many are in flight.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Where a dense thread lets the next step in: after its loads, but after its
+// stores in the FP64 steps, whose blocks compute so long that a next step's
+// blocks beside them settle unevenly.  us a step, no dependent launch / at the
+// kernel's start / after the loads / after the stores: FP32 channel 20x18x16
+// 2.29 / 1.66 / 1.73 / 1.99, 40x33x27 2.68 / 2.62 / 2.06 / 2.31, 60x57x56 5.4 /
+// 4.5 / 4.7 / 4.8; fast FP64 40x33x27 5.9 / 7.8 / 5.3 / 5.5; FP64 40x33x27 13.0 /
+// 18.8 / 12.8 / 12.5, 4x34x4 7.9 / 8.1 / 7.8 / 7.6
+template <class PH> constexpr bool late_trigger = uses_host_consts<PH>::value || uses_force_density<PH>::value;
+
+// launches kernel with that attribute
+template <class... P, class... A>
+cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // dense (interior / plain bounce-back / periodic) nodes
 // ---------------------------------------------------------------------------
@@ -225,6 +259,7 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
     if (cls >= CLS_SPECIAL) return;
     // the link mask matters only to the pull-push step of wall nodes
     const uint32_t m = (PSTEP && cls == CLS_WALL) ? __ldg(a.nmask + n) : 0u;
+    wait_previous();
 
     S *__restrict__ f = (S *)a.f;
     const IT Np = (IT)a.Np;
@@ -265,6 +300,7 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
       });
     };
     gather(fv);
+    if (!late_trigger<PH>) let_next_start();
 
     C ux, uy, uz, rho;
     if constexpr (uses_force_density<PH>::value) {
@@ -360,6 +396,7 @@ __device__ __forceinline__ void special_node(const StepArgs &a, int b) {
     const int64_t pn = a.sp_cnode ? __ldg(a.sp_cnode + t) : n;
     const int64_t PNp = a.sp_cnode ? a.Npc : Np;
     C *spden = (C *)a.sp_den;
+    wait_previous();
     const C dprev = spden[t];
     C fv[Q];
 
@@ -449,6 +486,7 @@ __device__ __forceinline__ void sparse_node(const StepArgs &a, int b) {
     using C = typename ST::C;
     const uint32_t m = (uint32_t)b * (blockDim.x * blockDim.y) + (threadIdx.y * blockDim.x + threadIdx.x);
     if (m >= (uint64_t)a.Nc) return;
+    wait_previous(); // also for the packed classes, which a kernel wrote
     S *__restrict__ f = (S *)a.f;
     const uint32_t Npc = (uint32_t)a.Npc; // 19 * Npc < 2^32 (checked by the host)
     // packed class and mask: they come with the site's index, not after it, and
@@ -493,6 +531,7 @@ __device__ __forceinline__ void sparse_node(const StepArgs &a, int b) {
         else e = (uint32_t)OPP(q) * Npc + nbr.template operator()<OPP(q)>();
         fv[q] = bulk_ld<ST, PH, q>(f + e);
     });
+    let_next_start();
     if (!PSTEP && cls >= CLS_SPECIAL) return;
     C ux, uy, uz;
     C ax, ay, az;
@@ -601,6 +640,7 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_STEP) lbm_step_kernel(cons
     } else {
         special_node<ST, PH, PSTEP, ACCF>(a, (int)blockIdx.x);
     }
+    if (late_trigger<PH>) let_next_start();
 }
 
 template <class ST, class PH, bool PSTEP, bool ACCF>
@@ -614,7 +654,8 @@ __global__ void __launch_bounds__(128, PSTEP ? JLB_MIN_BLOCKS_SPARSE : JLB_MIN_B
 
 template <class ST, template <int> class PH>
 int launch_step_sparse_impl(const StepArgs &a, int scheme, bool pstep, bool accf, int blocks, cudaStream_t st) {
-#define JLB_SL(SCH, P, A) lbm_step_sparse_kernel<ST, PH<SCH>, P, A><<<blocks, 128, 0, st>>>(a)
+    cudaError_t r = cudaSuccess;
+#define JLB_SL(SCH, P, A) r = launch_step(lbm_step_sparse_kernel<ST, PH<SCH>, P, A>, dim3(blocks), dim3(128), 0, st, a)
 #define JLB_SS(SCH)                                                          \
     if (pstep) { if (accf) JLB_SL(SCH, true, true); else JLB_SL(SCH, true, false); } \
     else { if (accf) JLB_SL(SCH, false, true); else JLB_SL(SCH, false, false); }
@@ -623,17 +664,19 @@ int launch_step_sparse_impl(const StepArgs &a, int scheme, bool pstep, bool accf
     else { JLB_SS(SCH_REG) }
 #undef JLB_SS
 #undef JLB_SL
-    return (int)cudaGetLastError();
+    const cudaError_t l = cudaGetLastError();
+    return (int)(r != cudaSuccess ? r : l);
 }
 
 template <class ST, template <int> class PH>
 int launch_step_impl(const StepArgs &a, int scheme, bool pstep, bool accf, int blocks, cudaStream_t st) {
     dim3 blk(a.bx, a.by), grd(blocks);
     const bool i64 = a.Np * 19 > 0x7fffffffLL;
+    cudaError_t r = cudaSuccess;
 #define JLB_L(SCH, P, A)                                                                 \
     do {                                                                                 \
-        if (i64) lbm_step_kernel<ST, PH<SCH>, P, A, int64_t><<<grd, blk, 0, st>>>(a);    \
-        else lbm_step_kernel<ST, PH<SCH>, P, A, int32_t><<<grd, blk, 0, st>>>(a);        \
+        r = i64 ? launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int64_t>, grd, blk, 0, st, a)   \
+                : launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int32_t>, grd, blk, 0, st, a);  \
     } while (0)
 #define JLB_S(SCH)                                   \
     if (pstep) { if (accf) JLB_L(SCH, true, true); else JLB_L(SCH, true, false); } \
@@ -643,7 +686,8 @@ int launch_step_impl(const StepArgs &a, int scheme, bool pstep, bool accf, int b
     else { JLB_S(SCH_REG) }
 #undef JLB_S
 #undef JLB_L
-    return (int)cudaGetLastError();
+    const cudaError_t l = cudaGetLastError();
+    return (int)(r != cudaSuccess ? r : l);
 }
 
 } // namespace jlb

@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_TMA) lbm_step_tma_kernel(c
         mbar_fence_init();
     }
     __syncthreads();
+    wait_previous();
 
     S *__restrict__ f = (S *)a.f;
     const int32_t Np = (int32_t)a.Np;
@@ -227,6 +228,7 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_TMA) lbm_step_tma_kernel(c
         }
         __syncthreads(); // buffer `cur` is free for the copies issued next round
     }
+    let_next_start();
 }
 
 // ---------------------------------------------------------------------------
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_H2) lbm_step_tma_h2_kernel
         mbar_fence_init();
     }
     __syncthreads();
+    wait_previous();
     __half *__restrict__ f = (__half *)a.f;
     const int32_t Np = (int32_t)a.Np;
     int tile = blockIdx.x;
@@ -347,20 +350,23 @@ __global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_H2) lbm_step_tma_h2_kernel
         }
         __syncthreads(); // buffer `cur` is free for the copies issued next round
     }
+    let_next_start();
 }
 
 template <template <int> class PH>
 int launch_step_tma_h2_impl(const StepArgs &a, int scheme, bool accf, int grid, int ntiles, int kb2,
                             int nspecial_blocks, int *err, cudaStream_t st) {
     const size_t smem = 2 * (size_t)H2Geom::STAGE * sizeof(__half);
-#define JLB_H(SCH, A) lbm_step_tma_h2_kernel<PH<SCH>, A><<<grid, 128, smem, st>>>(a, ntiles, kb2, nspecial_blocks, err)
+    cudaError_t r = cudaSuccess;
+#define JLB_H(SCH, A) r = launch_step(lbm_step_tma_h2_kernel<PH<SCH>, A>, dim3(grid), dim3(128), smem, st, a, ntiles, kb2, nspecial_blocks, err)
 #define JLB_HS(SCH) if (accf) JLB_H(SCH, true); else JLB_H(SCH, false);
     if (scheme == SCH_BGK) { JLB_HS(SCH_BGK) }
     else if (scheme == SCH_TRT) { JLB_HS(SCH_TRT) }
     else { JLB_HS(SCH_REG) }
 #undef JLB_HS
 #undef JLB_H
-    return (int)cudaGetLastError();
+    const cudaError_t l = cudaGetLastError();
+    return (int)(r != cudaSuccess ? r : l);
 }
 
 template <template <int> class PH> int tma_h2_blocks_per_sm(int scheme) {
@@ -379,7 +385,8 @@ int launch_step_tma_impl(const StepArgs &a, int scheme, bool pstep, bool accf, i
     using G = TmaGeom<typename ST::S>;
     const size_t smem = 2 * (size_t)G::STAGE * sizeof(typename ST::S);
     static_assert(2 * G::STAGE * sizeof(typename ST::S) <= 48 * 1024, "staging must fit the default smem limit");
-#define JLB_T(SCH, P, A) lbm_step_tma_kernel<ST, PH<SCH>, P, A><<<grid, 128, smem, st>>>(a, ntiles, nspecial_blocks, err)
+    cudaError_t r = cudaSuccess;
+#define JLB_T(SCH, P, A) r = launch_step(lbm_step_tma_kernel<ST, PH<SCH>, P, A>, dim3(grid), dim3(128), smem, st, a, ntiles, nspecial_blocks, err)
 #define JLB_TS(SCH)                                                                                      \
     if (pstep) { if (accf) JLB_T(SCH, true, true); else JLB_T(SCH, true, false); }                       \
     else { if (accf) JLB_T(SCH, false, true); else JLB_T(SCH, false, false); }
@@ -388,7 +395,8 @@ int launch_step_tma_impl(const StepArgs &a, int scheme, bool pstep, bool accf, i
     else { JLB_TS(SCH_REG) }
 #undef JLB_TS
 #undef JLB_T
-    return (int)cudaGetLastError();
+    const cudaError_t l = cudaGetLastError();
+    return (int)(r != cudaSuccess ? r : l);
 }
 
 } // namespace jlb
