@@ -23,14 +23,15 @@ COMMON = ["-std=c++20", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "-I", CSRC, "-I", INCLUDE]
 HOST_FLAGS = ["-x", "cu", "-Xcompiler", "-fopenmp", "-Xcompiler", "-ffp-contract=off"]
 UNITS = {
-    # 4 resident blocks (128 registers): the FP64 pipe and the integer pipes
-    # work for different warps at once.  At 3 / 4 / 5 blocks, us a step: 128^3
-    # TRT cavity 463 / 452 / 444, 4x34x4 channel 7.3 / 7.9 / 8.5
-    "lbm_fp64.cu": ["-fmad=false", "-DJLB_MIN_BLOCKS=4"],
+    # the FP64 pipe and the integer pipes work for different warps at once: 5
+    # resident blocks (96 registers), but 3 (168, no spills) where a launch has
+    # no more than that.  At 3 / 4 / 5 blocks, us a step: 128^3 TRT cavity 463 /
+    # 452 / 444, regularized 389 / 366 / 359, 4x34x4 channel 7.4 / 7.6 / 8.5
+    "lbm_fp64.cu": ["-fmad=false", "-DJLB_MIN_BLOCKS=5", "-DJLB_MIN_BLOCKS_FEW=3"],
     # the fast FP64 step: contracted on purpose.  5 resident blocks (96
     # registers, a few spilled): 256^3 TRT cavity 1390 / 1197 / 1178 us a step
-    # at 3 / 4 / 5
-    "lbm_fp64fast.cu": ["-DJLB_MIN_BLOCKS=5"],
+    # at 3 / 4 / 5; 3 where a launch has no more (40x33x27: 5.57 / 5.56 / 6.01)
+    "lbm_fp64fast.cu": ["-DJLB_MIN_BLOCKS=5", "-DJLB_MIN_BLOCKS_FEW=3"],
     # resident 128-thread blocks per SM.  The direct steps are latency-bound
     # on HBM: 8 blocks (<= 64 registers, 32 warps) keep more loads in flight
     # than 6 or 7, even where a few registers spill.  The persistent staged L

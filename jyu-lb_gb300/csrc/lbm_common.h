@@ -140,6 +140,7 @@ struct StepArgs {
     // dense-node grid
     int bx, by, kblocks;  // block shape and k-blocks per row-block
     int nb_dense;         // number of dense blocks; the rest are boundary blocks
+    int few;              // 1: a launch has at most three blocks per SM
     int rev;              // 1: dense blocks (tiles) run from the last to the first
     int b0;               // first dense block of this launch (a launch may cover a slab)
     int pf;               // L2 prefetch distance in dense blocks (0: none): block b

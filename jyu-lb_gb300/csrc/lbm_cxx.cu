@@ -205,8 +205,8 @@ int launch_cxx_typed(const StepArgs &a, bool pstep, bool accf, int blocks, cudaS
     using PH = PhysCxx<SCH, EQ2, FRC2>;
 #define JLB_CX(P, A)                                                                             \
     do {                                                                                         \
-        if (i64) lbm_step_kernel<StoreF64, PH, P, A, int64_t><<<grd, blk, 0, st>>>(a);           \
-        else lbm_step_kernel<StoreF64, PH, P, A, int32_t><<<grd, blk, 0, st>>>(a);               \
+        if (i64) lbm_step_kernel<StoreF64, PH, P, A, int64_t, JLB_MIN_BLOCKS_STEP><<<grd, blk, 0, st>>>(a); \
+        else lbm_step_kernel<StoreF64, PH, P, A, int32_t, JLB_MIN_BLOCKS_STEP><<<grd, blk, 0, st>>>(a);     \
     } while (0)
     if (pstep) { if (accf) JLB_CX(true, true); else JLB_CX(true, false); }
     else { if (accf) JLB_CX(false, true); else JLB_CX(false, false); }

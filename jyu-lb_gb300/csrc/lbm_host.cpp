@@ -632,6 +632,7 @@ StepArgs make_args(const jlb_solver *s, int write_moments) {
     }
     a.pf = s->pf_blocks;
     a.M = s->M;
+    a.few = (int64_t)a.nb_dense + special_blocks(a) <= (int64_t)3 * s->sms && 19 * s->Np <= 0x7fffffffLL;
     a.sp_node = s->d_sp_node; a.sp_info = s->d_sp_info;
     a.sp_rd = s->d_sp_rd; a.sp_wr = s->d_sp_wr;
     a.sp_lw = s->d_sp_lw; a.sp_bc = s->d_sp_bc;
@@ -719,6 +720,7 @@ void choose_kernel(jlb_solver *s) {
             cudaGetLastError();
             sms = 0;
         }
+        s->sms = sms;
         // only where the populations do not stay in L2 between steps (a
         // lattice that fits gains nothing and pays for the instructions)
         int l2 = 0;

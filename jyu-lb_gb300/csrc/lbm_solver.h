@@ -106,6 +106,7 @@ struct jlb_solver {
     bool use_h2 = false;  // FP16: staged local step with two sites per thread
     int h2_grid = 0;
     int *d_err = nullptr; // set by a kernel whose bounded wait timed out
+    int sms = 0;          // multiprocessors of the device
     int pf_blocks = 0;    // L2 prefetch distance of the direct step kernel (dense blocks)
     uint64_t args_version = 1, graph_version[2] = {0, 0};
 };

@@ -625,8 +625,13 @@ __device__ __forceinline__ void prefetch_block(const StepArgs &a, int b, int lan
 #ifndef JLB_MIN_BLOCKS_SPARSE_L
 #define JLB_MIN_BLOCKS_SPARSE_L JLB_MIN_BLOCKS_SPARSE
 #endif
-template <class ST, class PH, bool PSTEP, bool ACCF, class IT>
-__global__ void __launch_bounds__(128, JLB_MIN_BLOCKS_STEP) lbm_step_kernel(const StepArgs a) {
+// a second bound for grids that leave every block a third of an SM's registers
+// anyway (StepArgs::few); 0: none
+#ifndef JLB_MIN_BLOCKS_FEW
+#define JLB_MIN_BLOCKS_FEW 0
+#endif
+template <class ST, class PH, bool PSTEP, bool ACCF, class IT, int MINB>
+__global__ void __launch_bounds__(128, MINB) lbm_step_kernel(const StepArgs a) {
     // boundary nodes first: their chain of index loads, Zou-He sums and
     // collision is the longest, and at the end of the grid it was a tail (us a
     // step, last / first: FP32 duct 200x90x75 36.6 / 32.6, FP32 cavity 60x57x56
@@ -672,11 +677,16 @@ template <class ST, template <int> class PH>
 int launch_step_impl(const StepArgs &a, int scheme, bool pstep, bool accf, int blocks, cudaStream_t st) {
     dim3 blk(a.bx, a.by), grd(blocks);
     const bool i64 = a.Np * 19 > 0x7fffffffLL;
+    constexpr int FEW = JLB_MIN_BLOCKS_FEW ? JLB_MIN_BLOCKS_FEW : JLB_MIN_BLOCKS_STEP;
     cudaError_t r = cudaSuccess;
 #define JLB_L(SCH, P, A)                                                                 \
     do {                                                                                 \
-        r = i64 ? launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int64_t>, grd, blk, 0, st, a)   \
-                : launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int32_t>, grd, blk, 0, st, a);  \
+        if (JLB_MIN_BLOCKS_FEW && a.few)                                                         \
+            r = launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int32_t, FEW>, grd, blk, 0, st, a); \
+        else if (i64)                                                                            \
+            r = launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int64_t, JLB_MIN_BLOCKS_STEP>, grd, blk, 0, st, a); \
+        else                                                                                     \
+            r = launch_step(lbm_step_kernel<ST, PH<SCH>, P, A, int32_t, JLB_MIN_BLOCKS_STEP>, grd, blk, 0, st, a); \
     } while (0)
 #define JLB_S(SCH)                                   \
     if (pstep) { if (accf) JLB_L(SCH, true, true); else JLB_L(SCH, true, false); } \
