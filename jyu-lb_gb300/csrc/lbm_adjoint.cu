@@ -510,6 +510,7 @@ template <class ST, int SCH, bool PSTEP, bool SEED, class IT>
 __global__ void __launch_bounds__(128, adj_min_blocks<ST, SEED>()) adjoint_step_kernel(const AdjArgs A) {
     using C = typename ST::C;
     C pg[5] = {0, 0, 0, 0, 0};
+    wait_previous(); // every thread: the block's slot is added to below
     // boundary sites first (the longer chain); a block's slot does not depend
     // on the launch order: dense blocks, then boundary blocks
     const int nsp = (int)gridDim.x - A.s.nb_dense;
@@ -517,6 +518,7 @@ __global__ void __launch_bounds__(128, adj_min_blocks<ST, SEED>()) adjoint_step_
     const int b = n < 0 ? A.s.nb_dense + (int)blockIdx.x : A.s.rev ? A.s.nb_dense - 1 - n : n;
     if (b < A.s.nb_dense) adjoint_dense_sites<ST, SCH, PSTEP, SEED, IT>(A, b, pg);
     else adjoint_boundary_sites<ST, SCH, PSTEP, SEED>(A, b - A.s.nb_dense, pg);
+    let_next_start();
     block_sensitivities<C>(pg, A.part + 5 * (int64_t)b);
 }
 
@@ -526,9 +528,11 @@ int launch_adjoint_typed(const AdjArgs &A, cudaStream_t st) {
     const int blocks = adjoint_blocks(a);
     if (blocks == 0) return 0;
     const dim3 blk(a.bx, a.by), grd(blocks);
-    if (a.Np * 19 > 0x7fffffffLL) adjoint_step_kernel<ST, SCH, PSTEP, SEED, int64_t><<<grd, blk, 0, st>>>(A);
-    else adjoint_step_kernel<ST, SCH, PSTEP, SEED, int32_t><<<grd, blk, 0, st>>>(A);
-    return (int)cudaGetLastError();
+    const cudaError_t r = a.Np * 19 > 0x7fffffffLL
+                              ? launch_step(adjoint_step_kernel<ST, SCH, PSTEP, SEED, int64_t>, grd, blk, 0, st, A)
+                              : launch_step(adjoint_step_kernel<ST, SCH, PSTEP, SEED, int32_t>, grd, blk, 0, st, A);
+    const cudaError_t l = cudaGetLastError();
+    return (int)(r != cudaSuccess ? r : l);
 }
 
 template <class ST, int SCH>
