@@ -104,12 +104,12 @@ __device__ __forceinline__ int axcomp(int q, int ax) { return ax == 0 ? CX(q) : 
 // mu the adjoint w.r.t. the pre-Zou-He populations and adds the adjoint of the
 // face data: du (boundary velocity; a FIXED_DEN face uses its tangential
 // components) and dden (density of a FIXED_DEN face).
-template <class C, bool SHIFTED>
-__device__ void zh_adjoint(int fc, int kind, double den, double ux, double uy, double uz, const C *gp, C *mu,
-                           double *du, double &dden) {
-    const int ax = fc >> 1;
-    const bool high = fc & 1;
-    const int in_sign = high ? -1 : 1; // normal component of the unknown populations
+template <class C, bool SHIFTED, int fc>
+__device__ __forceinline__ void zh_adjoint(int kind, double den, double ux, double uy, double uz, const C *gp, C *mu,
+                                           double *du, double &dden) {
+    constexpr int ax = fc >> 1;
+    constexpr bool high = fc & 1;
+    constexpr int in_sign = high ? -1 : 1; // normal component of the unknown populations
     // S = sum of populations with zero normal component + 2 * sum leaving
     C S = SHIFTED ? (C)1 : (C)0;
 #pragma unroll
@@ -129,7 +129,8 @@ __device__ void zh_adjoint(int fc, int kind, double den, double ux, double uy, d
         zh_assign<C>(fc, (C)0, (C)0, (C)0, e);
         C acc = 0;
 #pragma unroll
-        for (int p = 0; p < Q; ++p) acc += mu[p] * e[p];
+        for (int p = 0; p < Q; ++p)
+            if (e[p] != (C)0) acc += mu[p] * e[p];
         lam[q] = acc;
     }
     C dj[3];
@@ -141,7 +142,8 @@ __device__ void zh_adjoint(int fc, int kind, double den, double ux, double uy, d
         zh_assign<C>(fc, a == 0 ? (C)1 : (C)0, a == 1 ? (C)1 : (C)0, a == 2 ? (C)1 : (C)0, e);
         C acc = 0;
 #pragma unroll
-        for (int p = 0; p < Q; ++p) acc += mu[p] * e[p];
+        for (int p = 0; p < Q; ++p)
+            if (e[p] != (C)0) acc += mu[p] * e[p];
         dj[a] = acc;
     }
     C dS;
@@ -350,17 +352,12 @@ template <class C> __device__ __forceinline__ void block_sensitivities(C *pg, do
     }
 }
 
-// resident 128-thread blocks per SM asked of the register allocator (the
-// seeding launch, which also forms the loss gradient, gets one fewer)
+// resident 128-thread blocks per SM asked of the register allocator: 200 steps
+// of the 256x64x64 channel, TRT, at 5 / 6 / 7: 12.87 / 13.24 / 13.26 ms
 #ifndef JLB_ADJ_MIN_BLOCKS
-#define JLB_ADJ_MIN_BLOCKS 6
+#define JLB_ADJ_MIN_BLOCKS 5
 #endif
-#ifndef JLB_ADJ_MIN_BLOCKS_SEED
-#define JLB_ADJ_MIN_BLOCKS_SEED 5
-#endif
-template <class ST, bool SEED> constexpr int adj_min_blocks() {
-    return ST::shifted ? (SEED ? JLB_ADJ_MIN_BLOCKS_SEED : JLB_ADJ_MIN_BLOCKS) : 1;
-}
+template <class ST> constexpr int adj_min_blocks() { return ST::shifted ? JLB_ADJ_MIN_BLOCKS : 1; }
 
 // Dense sites.  Their collision inputs are gathered from the state before the
 // step (A.snap) exactly as the forward step gathers them; the adjoint of the
@@ -469,22 +466,25 @@ __device__ __forceinline__ void adjoint_boundary_sites(const AdjArgs &A, int b, 
         }
         const uint32_t info = __ldg(a.sp_info + t);
         const uint32_t faces = (info >> SP_FACE_SHIFT) & 0x3Fu;
-        // faces were applied in increasing order, so transpose in decreasing
-        int slots[6], nf = 0;
-        for (int fc = 0; fc < 6; ++fc)
-            if (faces & (1u << fc)) slots[fc] = nf++;
-        for (int fc = 5; fc >= 0; --fc) {
-            if (!(faces & (1u << fc))) continue;
-            const double *bcd = a.sp_bc + (int64_t)(4 * slots[fc]) * M + t;
+        // faces were applied in increasing order, so transpose in decreasing; the
+        // face is a template parameter, so that the unit vectors the transpose is
+        // read from fold to the few terms that are not zero (with the face in a
+        // loop, this chain was most of a small problem's step: 100x30x33, 100
+        // steps, 1.53 -> 0.94 ms)
+        Unroll<0, 6>::run([&]<int r>() {
+            constexpr int fc = 5 - r;
+            if (!(faces & (1u << fc))) return;
+            const int slot = __popc(faces & ((1u << fc) - 1u));
+            const double *bcd = a.sp_bc + (int64_t)(4 * slot) * M + t;
             double du[3] = {0, 0, 0}, dden = 0.0;
-            zh_adjoint<C, ST::shifted>(fc, a.bc[fc], bcd[0], bcd[M], bcd[2 * (int64_t)M], bcd[3 * (int64_t)M], g,
-                                       li, du, dden);
+            zh_adjoint<C, ST::shifted, fc>(a.bc[fc], bcd[0], bcd[M], bcd[2 * (int64_t)M], bcd[3 * (int64_t)M], g,
+                                           li, du, dden);
             // one thread per boundary site: plain adds are race-free
             if (A.grad_bc && ((A.param_faces >> fc) & 1u)) {
                 A.grad_bc[t] += dden;
                 for (int c = 0; c < 3; ++c) A.grad_bc[(int64_t)(1 + c) * M + t] += du[c];
             }
-        }
+        });
         if (lam_den) {
             // Ladd's term of a moving link, g_q = f + 6 w_q den_prev (c_q . u_wall),
             // passes its adjoint to the density of the previous step
@@ -507,7 +507,7 @@ int adjoint_blocks(const StepArgs &a) { return a.nb_dense + special_blocks(a); }
 // One step of the reverse sweep: the first blocks take the boundary sites,
 // the last nb_dense the dense sites (disjoint address sets, as in the forward step).
 template <class ST, int SCH, bool PSTEP, bool SEED, class IT>
-__global__ void __launch_bounds__(128, adj_min_blocks<ST, SEED>()) adjoint_step_kernel(const AdjArgs A) {
+__global__ void __launch_bounds__(128, adj_min_blocks<ST>()) adjoint_step_kernel(const AdjArgs A) {
     using C = typename ST::C;
     C pg[5] = {0, 0, 0, 0, 0};
     wait_previous(); // every thread: the block's slot is added to below
