@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(BLOCK, JLB_BATCH_WARPS * 32 / BLOCK)
     using PH = PhysSh<SCH>;
     using C = float;
     const int b = (int)blockIdx.x;
-    const int t = a.rev ? a.ntiles - 1 - b : b;
+    const int t = a.tile0 + (a.rev ? a.ntiles - 1 - b : b);
     if (a.pf && threadIdx.x < 32 && b + a.pf < a.ntiles)
         batch_prefetch<PSTEP, BLOCK>(a, a.rev ? t - a.pf : t + a.pf, (int)threadIdx.x);
     const int d = __ldg(a.tile_dom + t);
@@ -173,8 +173,10 @@ int launch_batch_step(const BatchArgs &a, int scheme, bool pstep, int block, int
 // rates, body force and face kinds of each node's domain.
 template <int SCH, bool PSTEP>
 __global__ void __launch_bounds__(128) lbm_batch_special_kernel(const BatchArgs a) {
-    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (t >= a.Msp) return;
+    // whole blocks of the tables: the first may begin before the launch's nodes
+    const int b = a.sp0 / (int)blockDim.x + (int)blockIdx.x;
+    const int t = b * (int)blockDim.x + (int)threadIdx.x;
+    if (t < a.sp0 || t >= a.sp1) return;
     const BatchDomain &D = a.dom[__ldg(a.sp_dom + t)];
     StepArgs s{};
     s.f = a.f;
@@ -198,12 +200,12 @@ __global__ void __launch_bounds__(128) lbm_batch_special_kernel(const BatchArgs 
         s.gf[c] = D.g[c];
     }
     for (int f = 0; f < 6; ++f) s.bc[f] = D.bc[f];
-    special_node<StoreF32, PhysSh<SCH>, PSTEP, false>(s, (int)blockIdx.x);
+    special_node<StoreF32, PhysSh<SCH>, PSTEP, false>(s, b);
 }
 
 int launch_batch_special(const BatchArgs &a, int scheme, bool pstep, cudaStream_t st) {
-    if (a.Msp <= 0) return 0;
-    const unsigned blocks = (unsigned)((a.Msp + 127) / 128);
+    if (a.sp1 <= a.sp0) return 0;
+    const unsigned blocks = (unsigned)((a.sp1 + 127) / 128 - a.sp0 / 128);
 #define JLB_BS2(SCH) \
     if (pstep) lbm_batch_special_kernel<SCH, true><<<blocks, 128, 0, st>>>(a); \
     else lbm_batch_special_kernel<SCH, false><<<blocks, 128, 0, st>>>(a);

@@ -38,7 +38,7 @@ struct BatchArgs {
     float *dprev;          // previous-step rho - 1 (MOVING nodes)
     float *den, *ux, *uy, *uz;
     int write_moments;
-    int ntiles;            // tiles of the launch
+    int tile0, ntiles;     // first tile and tiles of the launch
     int rev;               // 1: tiles run from the last to the first
     int pf;                // L2 prefetch distance in tiles: the block of tile t
                            // prefetches the rows tile t + pf reads (0: none)
@@ -46,6 +46,7 @@ struct BatchArgs {
     // single-domain table layout ([19][Msp] element indices into f, Zou-He
     // data fixed at set-up) with the domain of each
     int Msp;
+    int sp0, sp1;          // boundary nodes [sp0, sp1) of the launch
     const int32_t *sp_dom;
     const int64_t *sp_node, *sp_rd, *sp_wr;
     const uint32_t *sp_info;

@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "jyulb_gb300.h"
@@ -40,6 +41,10 @@ struct jlb_batch {
     double tune_ms[3] = {0, 0, 0}; // per-step time of blocks 64 / 128 / 256
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
     int GK = 32;
+    // runs of domains [first, last) advanced one after another, each for all
+    // steps of a call; group_bytes bounds their populations
+    std::vector<std::pair<int, int>> groups;
+    double group_bytes = 0;
     // boundary nodes of domains with Zou-He or symmetric faces (device
     // tables in the single-domain layout, element indices into f)
     int Msp = 0;
@@ -90,7 +95,10 @@ BatchArgs batch_args(const jlb_batch *b, int write_moments) {
     a.dprev = b->dprev;
     a.den = b->mom[0]; a.ux = b->mom[1]; a.uy = b->mom[2]; a.uz = b->mom[3];
     a.write_moments = write_moments;
+    a.tile0 = 0;
     a.ntiles = b->ntiles;
+    a.sp0 = 0;
+    a.sp1 = b->Msp;
     a.pf = b->pf;
     a.Msp = b->Msp;
     a.sp_dom = b->d_sp_dom;
@@ -132,15 +140,22 @@ int batch_tiles(jlb_batch *b, int block) {
     return JLB_OK;
 }
 
-int batch_launch(jlb_batch *b, bool pstep, int write_moments) {
+// one step of the domains [d0, d1)
+int batch_launch(jlb_batch *b, bool pstep, int write_moments, int d0, int d1) {
     BatchArgs a = batch_args(b, write_moments);
+    a.tile0 = b->dom[d0].first_tile;
+    a.ntiles = (d1 < b->ndom ? b->dom[d1].first_tile : b->ntiles) - a.tile0;
+    a.sp0 = b->sp_first.empty() ? 0 : b->sp_first[d0];
+    a.sp1 = b->sp_first.empty() ? 0 : b->sp_first[d1];
+    // a group that stays in the L2 needs no prefetch into it
+    if (b->groups.size() > 1 && 76.0 * (double)a.ntiles * b->block <= b->group_bytes + 76.0 * 128 * (d1 - d0)) a.pf = 0;
     // from the end where the last step left its lines in the L2: 32 channels
     // (0.9 GB) 254.7 -> 248.2 us a step
     a.rev = !pstep;
-    int r = launch_batch_step(a, b->scheme, pstep, b->block, b->ntiles, b->st);
+    int r = launch_batch_step(a, b->scheme, pstep, b->block, a.ntiles, b->st);
     if (r) return bfail(b, JLB_ERR_CUDA, std::string("batch step: ") + cudaGetErrorString((cudaError_t)r));
     ++b->launches;
-    if (b->Msp > 0) {
+    if (a.sp1 > a.sp0) {
         r = launch_batch_special(a, b->scheme, pstep, b->st);
         if (r) return bfail(b, JLB_ERR_CUDA, std::string("batch boundary nodes: ") + cudaGetErrorString((cudaError_t)r));
         ++b->launches;
@@ -150,6 +165,15 @@ int batch_launch(jlb_batch *b, bool pstep, int write_moments) {
 
 int batch_run(jlb_batch *b, uint32_t n, bool write_last) {
     uint32_t plain = write_last && n > 0 ? n - 1 : n;
+    if (b->groups.size() > 1) {
+        for (const auto &g : b->groups)
+            for (uint32_t t = 0; t < n; ++t) {
+                int r = batch_launch(b, ((b->parity + t) & 1) == 0, write_last && t + 1 == n, g.first, g.second);
+                if (r) return r;
+            }
+        b->parity ^= (int)(n & 1);
+        return JLB_OK;
+    }
     while (graphs_enabled() && plain >= (uint32_t)b->GK) {
         const int p = b->parity;
         if (!b->gexec[p]) {
@@ -157,7 +181,7 @@ int batch_run(jlb_batch *b, uint32_t n, bool write_last) {
             BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
             int par = p, rr = JLB_OK;
             for (int t = 0; t < b->GK && rr == JLB_OK; ++t) {
-                rr = batch_launch(b, par == 0, 0);
+                rr = batch_launch(b, par == 0, 0, 0, b->ndom);
                 par ^= 1;
             }
             cudaError_t ce = cudaStreamEndCapture(b->st, &g);
@@ -174,12 +198,12 @@ int batch_run(jlb_batch *b, uint32_t n, bool write_last) {
         if (b->GK & 1) b->parity ^= 1;
     }
     for (uint32_t t = 0; t < plain; ++t) {
-        int r = batch_launch(b, b->parity == 0, 0);
+        int r = batch_launch(b, b->parity == 0, 0, 0, b->ndom);
         if (r) return r;
         b->parity ^= 1;
     }
     if (write_last && n > 0) {
-        int r = batch_launch(b, b->parity == 0, 1);
+        int r = batch_launch(b, b->parity == 0, 1, 0, b->ndom);
         if (r) return r;
         b->parity ^= 1;
     }
@@ -210,9 +234,9 @@ int batch_autotune(jlb_batch *b) {
     for (int c = 0; c < 3; ++c) {
         int r = batch_tiles(b, cand[c]);
         if (r) return r;
-        for (int t = 0; t < 2; ++t) if ((r = batch_launch(b, t == 0, 0))) return r;
+        for (int t = 0; t < 2; ++t) if ((r = batch_launch(b, t == 0, 0, 0, b->ndom))) return r;
         cudaEventRecord(e0, b->st);
-        for (int t = 0; t < 4; ++t) if ((r = batch_launch(b, t % 2 == 0, 0))) return r;
+        for (int t = 0; t < 4; ++t) if ((r = batch_launch(b, t % 2 == 0, 0, 0, b->ndom))) return r;
         cudaEventRecord(e1, b->st);
         cudaEventSynchronize(e1);
         float ms = 0;
@@ -519,11 +543,30 @@ int jlb_batch_create(int32_t scheme, const jlb_domain *doms, int32_t ndom, void 
         b->pf_big = 19.0 * (double)b->Np * sizeof(float) > 2.0 * (double)l2;
         const char *e = std::getenv("JLB_BATCH_PF");
         if (e && e[0]) b->pf_tiles = std::max(0, std::atoi(e));
+        const char *eg = std::getenv("JLB_BATCH_GROUP");
+        b->group_bytes = eg && eg[0] ? 1e6 * std::atof(eg) : 0.65 * (double)l2;
     }
     const char *tune = std::getenv("JLB_BATCH_BLOCK");
     if (tune && tune[0]) r = batch_tiles(b, std::atoi(tune));
     else r = batch_autotune(b);
     if (r) return bail(r);
+    // Groups of consecutive domains whose populations stay in the L2 (129 MB)
+    // from step to step.  Domains do not touch each other, so a group may run
+    // all steps of a call before the next one begins; domains larger than that
+    // are groups by themselves.  32 channels (0.9 GB), us a step: all together
+    // 245.9, groups of 30 / 45 / 64 / 80 / 100 MB 229.6 / 215.8 / 212.2 / 209.2 /
+    // 209.8; 8 channels (76 MB): together 19.6, groups of 45 / 64 / 80 MB 23.0 /
+    // 21.2 / 19.6.  JLB_BATCH_GROUP=<MB> sets the size, 0 keeps them together.
+    double bytes = 0;
+    for (int d = 0; d < ndom; ++d) {
+        const double x = 19.0 * sizeof(float) * b->dom[d].n;
+        if (b->groups.empty() || (b->group_bytes > 0 && bytes + x > b->group_bytes)) {
+            b->groups.emplace_back(d, d);
+            bytes = 0;
+        }
+        b->groups.back().second = d + 1;
+        bytes += x;
+    }
     *out = b;
     return JLB_OK;
 }
