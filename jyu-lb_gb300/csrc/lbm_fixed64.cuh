@@ -7,7 +7,8 @@
 // 2^-61 the populations are exact (they are doubles of at least 2^-9), every
 // sum is exact, and a product rounds at 2^-62, where a double of a population's
 // size rounds at 2^-58 or above: the collision loses less than FP64 arithmetic
-// does, and only the store rounds to 53 bits.  One FP64 reciprocal is left.
+// does, and only the store rounds to 53 bits.  One FP64 reciprocal is left, for
+// the FP64 pipe has nothing else to do (soft64.cuh's: 128^3 145 -> 169 us a step).
 //
 // With pairs (m, p) of opposite populations, even part fe = f_p + f_m, odd
 // part fo = f_p - f_m, weight w and direction c of p, the update
