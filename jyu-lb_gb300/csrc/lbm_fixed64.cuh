@@ -72,8 +72,10 @@ inline FixConsts make_fix_consts(bool trt, bool reg, double we, double wo, const
 
 // f[19] in place; returns false (f undefined) where an operand leaves the
 // form's range: populations in [2^-9, 1/8) (rest: below 1) before and at least
-// 2^-9 after, density in [1/2, 3/2), |j + a den/2| < 1/4 per component.  With
-// `want`, mom receives den and the stored velocity u = j/den + a/2.
+// 2^-9 after, density in [1/2 + 2^-29, 3/2), |j + a den/2| < 1/4 per component.
+// (From 1/2 itself the reciprocal, with unit 2^-62, would reach 2^63: the
+// margin leaves digits() the 2^31 it adds.)  With `want`, mom receives den and
+// the stored velocity u = j/den + a/2.
 template <bool REG>
 S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool want, double *mom) {
     using namespace soft64;
@@ -111,7 +113,7 @@ S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool w
         sd[d] = digits(s[d]);
     }
     const bool bad = range > 5u || range9 > 8u || fast >= (1u << 28) ||
-                     (uint32_t)((uint64_t)den >> 32) - (1u << 28) >= (1u << 29);
+                     (uint32_t)((uint64_t)den >> 32) - ((1u << 28) + 1u) >= (1u << 29) - 1u;
     if (want) {
         mom[0] = dd;
 #pragma unroll

@@ -260,14 +260,19 @@ S64_FN double diff_to_double(uint64_t a, uint64_t b) {
 struct Fix2 {
     int32_t hi, lo;
 };
+// -2^63 <= x < 2^63 - 2^31
 S64_FN Fix2 digits(int64_t x) {
     Fix2 d;
     d.lo = (int32_t)(uint32_t)(uint64_t)x;
     d.hi = (int32_t)((x + 0x80000000ll) >> 32);
     return d;
 }
-// x y / 2^(64 - SH), rounded; |x| < 2^62, |y| < 2^62 and no overflow of the
-// result
+// x y / 2^(64 - SH), rounded, for operands that digits() holds with
+// |x| + |y| < 2^64 - 2^33 (the mixed products, below 2^31 (|x.hi| + |y.hi|) in
+// size, and the rounding term then stay below 2^63) and a result of less than
+// 2^63.  The collision's operands (lbm_fixed64.cuh), at most: 8 s 2^62 with the
+// reciprocal 2^63 - 2^34; momenta and velocities 2^61.2; 9 (fe - y) + b and
+// 6 fo - odd 2^62.6 with the rates 2^61.9; forces 2^60 with densities 2^61.6.
 template <int SH = 0> S64_FN int64_t mulq(const Fix2 &x, const Fix2 &y) {
     int64_t m = (int64_t)x.lo * y.hi + (0x80000000ll >> SH);
     m = (int64_t)x.hi * y.lo + m;
