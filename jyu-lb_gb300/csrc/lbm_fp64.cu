@@ -167,7 +167,7 @@ template <int SCH> struct Phys64 : Phys64Base {
 
     // The same update, with most of its operations on the integer pipes
     // (soft64.cuh): the same bits.  It needs populations in [2^-9, 1/4) (rest:
-    // up to 1/2), velocities that are zero or no smaller than 2^-400, and
+    // up to 1/2), velocities that are zero or in [2^-400, 2^8), and
     // projections whose even parts outweigh the odd ones; anything else sets
     // `bad` and leaves f undefined.
     __device__ static C collide_int(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz, bool &bad) {
@@ -253,17 +253,19 @@ template <int SCH> struct Phys64 : Phys64Base {
         uint32_t span = 0;
         int32_t apart = 1 << 30;
         project_int<SCH != SCH_REG>(h, k, f, span, apart);
-        // velocities are zero or at least 2^-400: their products are normal
-        uint32_t tiny = 0xffffffffu;
+        // velocities are zero or in [2^-400, 2^8): their products, and those
+        // with the force they bound, are normal.  An acceleration field may hold
+        // anything; mul() of a NaN or an infinity would be some finite number
+        uint32_t beyond = 0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const uint64_t u = bits(d == 0 ? ux : d == 1 ? uy : uz);
             const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
-            const uint32_t z = (u << 1) ? e : 0x7ffu;
-            tiny = tiny < z ? tiny : z;
+            const uint32_t z = (u << 1) ? e - (1023u - 400u) : 0u;
+            beyond = beyond > z ? beyond : z;
         }
         bad = range > 6u || range9 > 7u || least >= (1u << 31) - (1u << 21) || span > PROJ_SPAN || apart < 2 ||
-              tiny < 1023u - 400u;
+              beyond > 407u;
         return den;
     }
 

@@ -19,3 +19,19 @@ def test_fast_density_edges(scheme, rho, steps):
     run_both(lat, scheme, 0.05, (0, 0, 0), np.full(lat, rho), vel, None, steps, fast=True)
     # one velocity everywhere: every bulk site stays at the edge
     run_both(lat, scheme, 0.05, (0, 0, 0), np.full(lat, rho), np.full(lat + (3,), 0.03), None, steps, fast=True)
+
+
+# acceleration fields with sites far outside the range of the integer form's
+# products: NaN and infinities propagate as in the reference, everything else
+# keeps its bits
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 1e160, -1e100, 1e3, 300.0, 1e-200, 3e-310])
+@pytest.mark.parametrize("steps", [1, 2])
+def test_extreme_acceleration_field(scheme, value, steps):
+    rng = np.random.default_rng(22)
+    lat = (5, 6, 40)
+    den = 1 + 0.01 * rng.uniform(-1, 1, lat)
+    vel = 0.02 * rng.uniform(-1, 1, lat + (3,))
+    acc = np.where(rng.random(lat + (3,)) < 0.02, value, 1e-5 * rng.uniform(-1, 1, lat + (3,)))
+    acc[1, 1, 7] = value
+    run_both(lat, scheme, 0.05, (0, 2e-5, 0), den, vel, acc, steps)
