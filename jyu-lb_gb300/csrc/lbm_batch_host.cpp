@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -60,8 +61,11 @@ struct jlb_batch {
     int sms = 0;                     // multiprocessors of the device
     std::vector<int64_t> h_sp_node;  // [Msp] packed node of each boundary node
     std::vector<uint32_t> h_sp_info; // [Msp] its link / face bits
-    std::vector<uint8_t> h_cls;      // [Np] node classes, for the read-out
-    float *pinned = nullptr;         // page-locked staging of the moments' read-out
+    // read-out of the moments: node classes [Np] and page-locked staging, held
+    // by one read-out at a time
+    std::mutex readout;
+    std::vector<uint8_t> h_cls;
+    float *pinned = nullptr;
     size_t pinned_sites = 0;
     std::string err;
 };
@@ -635,18 +639,26 @@ int jlb_batch_set_bc(jlb_batch *b, int32_t d, const double *den, const double *v
 int jlb_batch_moments(jlb_batch *b, int32_t d, double *den, double *vel) {
     if (!b || d < 0 || d >= b->ndom || !den || !vel) return bfail(b, JLB_ERR_INVALID_ARG, "bad argument");
     const BatchDomain &B = b->dom[d];
+    // threads may read different domains at once: one at a time uses the
+    // staging (the copies share a stream anyway)
+    std::lock_guard<std::mutex> lock(b->readout);
     // page-locked staging of the largest domain's four moments, then one
     // parallel pass: pageable copies and a serial pass took 40 ms for 32
     // channels (11 M sites), more than 150 steps of them
     if (!b->pinned) {
         int32_t most = 0;
         for (const BatchDomain &x : b->dom) most = std::max(most, x.n);
-        BCK(cudaHostAlloc((void **)&b->pinned, (size_t)4 * most * sizeof(float), cudaHostAllocDefault));
-        b->pinned_sites = (size_t)most;
+        if (cudaHostAlloc((void **)&b->pinned, (size_t)4 * most * sizeof(float), cudaHostAllocDefault) == cudaSuccess) {
+            b->pinned_sites = (size_t)most;
+        } else {
+            cudaGetLastError();
+            b->pinned = nullptr;
+        }
     }
+    std::vector<float> own(b->pinned ? 0 : (size_t)4 * B.n); // no page-locked memory left
     float *h[4];
     for (int c = 0; c < 4; ++c) {
-        h[c] = b->pinned + (size_t)c * b->pinned_sites;
+        h[c] = b->pinned ? b->pinned + (size_t)c * b->pinned_sites : own.data() + (size_t)c * B.n;
         BCK(cudaMemcpyAsync(h[c], b->mom[c] + B.off, (size_t)B.n * sizeof(float), cudaMemcpyDeviceToHost, b->st));
     }
     if (b->h_cls.empty()) {
