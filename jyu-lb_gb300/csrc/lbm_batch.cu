@@ -60,12 +60,12 @@ __global__ void __launch_bounds__(BLOCK, JLB_BATCH_WARPS * 32 / BLOCK)
     if (l >= D.n) return;
     const int32_t n = D.off + l;
     const uint8_t cls = __ldg(a.ncls + n);
-    if (cls >= BCLS_SOLID) return;
     // rows of 19 * Np exceed 2^31 elements for large ensembles; each row
     // itself is indexed by a 32-bit site
     const uint32_t m = (PSTEP && cls != BCLS_PLAIN) ? __ldg(a.nmask + n) : 0u;
     const uint32_t mv = (cls == BCLS_MOVING) ? __ldg(a.mmask + n) : 0u;
     wait_previous();
+    if (cls >= BCLS_SOLID) return;
     C fv[Q];
     int32_t dI[3], dJ[3], dK[3];
     if (PSTEP) {

@@ -201,9 +201,10 @@ __device__ __forceinline__ int32_t split_div(int32_t l, int32_t d, float inv, in
 // Programmatic dependent launch between the steps of a stream or graph: a
 // step's blocks may become resident while the step before drains, work out
 // their sites and read the static classes, and wait here, before any
-// population, for that step to be complete and its stores visible.  Every
-// fluid site's thread waits, so a step cannot complete before the one before
-// it, however many are in flight.
+// population, for that step to be complete and its stores visible.  Threads
+// without a fluid site wait too: a launch none of whose threads waits (a slab of
+// boundary sites, a domain of solid ones) would complete before the one before
+// it, and whatever follows it in the stream would start too early.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -256,10 +257,10 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
     // element indices fit IT (int32 when 19 * Np < 2^31, chosen by the host)
     const IT n = (IT)row * a.nz + k;
     const uint8_t cls = __ldg(a.ncls + n);
-    if (cls >= CLS_SPECIAL) return;
     // the link mask matters only to the pull-push step of wall nodes
     const uint32_t m = (PSTEP && cls == CLS_WALL) ? __ldg(a.nmask + n) : 0u;
     wait_previous();
+    if (cls >= CLS_SPECIAL) return;
 
     S *__restrict__ f = (S *)a.f;
     const IT Np = (IT)a.Np;
