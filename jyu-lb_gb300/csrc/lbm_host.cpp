@@ -1444,6 +1444,17 @@ int jlb_evolve(jlb_solver *s, uint32_t tsteps, const double g[3], double *den, d
     using clk = std::chrono::steady_clock;
     auto since = [](clk::time_point a) { return std::chrono::duration<double>(clk::now() - a).count(); };
     const auto t_start = clk::now();
+    // den / vel belong to the call: a failing one waits for the halo rules'
+    // kernel (and slab copies) in flight on them before it returns
+    struct Settle {
+        jlb_solver *s;
+        bool done = false;
+        ~Settle() {
+            if (done) return;
+            if (s->st2) cudaStreamSynchronize(s->st2);
+            cudaStreamSynchronize(s->st);
+        }
+    } settle{s};
     if (int rh = halo_rules(s, den, vel, false)) return rh;
     // solid velocities: reclassify when any of them changed since the last call
     int changed = 0;
@@ -1499,6 +1510,7 @@ int jlb_evolve(jlb_solver *s, uint32_t tsteps, const double g[3], double *den, d
     if (s->use_tma && (r = check_kernel_error(s))) return r;
     s->host_t[4] += since(t1);
     s->host_t[5] += since(t_start);
+    settle.done = true; // the download has waited
     s->tot += tsteps;
     if (tot) *tot = s->tot;
     return JLB_OK;
