@@ -215,6 +215,8 @@ __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.w
 // 2.29 / 1.66 / 1.73 / 1.99, 40x33x27 2.68 / 2.62 / 2.06 / 2.31, 60x57x56 5.4 /
 // 4.5 / 4.7 / 4.8; fast FP64 40x33x27 5.9 / 7.8 / 5.3 / 5.5; FP64 40x33x27 13.0 /
 // 18.8 / 12.8 / 12.5, 4x34x4 7.9 / 8.1 / 7.8 / 7.6
+// In the fast FP64 step a site that takes the FP64 form computes as long as
+// those, and lets the next step in when it is done.
 template <class PH> constexpr bool late_trigger = uses_host_consts<PH>::value || uses_force_density<PH>::value;
 
 // launches kernel with that attribute
@@ -301,7 +303,7 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
       });
     };
     gather(fv);
-    if (!late_trigger<PH>) let_next_start();
+    if (!late_trigger<PH> && !(uses_fixed_point<PH>::value && !ACCF)) let_next_start();
 
     C ux, uy, uz, rho;
     if constexpr (uses_force_density<PH>::value) {
@@ -315,27 +317,43 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
     } else if constexpr (uses_host_consts<PH>::value) {
         const Force64 F = site_force64<ACCF>(a, n);
         bool bad = true;
-        if (a.k64.soft) rho = PH::collide_int(fv, F, a.k64, ux, uy, uz, bad);
+        const bool enter = a.k64.soft && PH::int_range(fv);
+        if (enter) rho = PH::collide_int(fv, F, a.k64, ux, uy, uz, bad);
         if (bad) {
-            // outside the integer form's range: nothing is stored yet, so the
-            // site is read again and takes the FP64 form
-            C g[Q], u[3];
-            gather(g);
-            rho = PH::collide_cold(g, F, a.k64, u);
-            ux = u[0]; uy = u[1]; uz = u[2];
-            Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
+            // outside the integer form's range: the site takes the FP64 form;
+            // nothing is stored yet, so what was overwritten is read again
+            if constexpr (PH::fallback_inline) {
+                if (enter) gather(fv);
+                rho = PH::collide(fv, F, a.k64, ux, uy, uz);
+            } else {
+                C g[Q], u[3];
+                if (enter) gather(g);
+                else Unroll<0, Q>::run([&]<int q>() { g[q] = fv[q]; });
+                rho = PH::collide_cold(g, F, a.k64, u);
+                ux = u[0]; uy = u[1]; uz = u[2];
+                Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
+            }
         }
     } else if constexpr (uses_fixed_point<PH>::value && !ACCF) {
         C mom[4];
         bool good = false;
-        if (a.fx.ok) good = collide_fixed<PH::regularized>(fv, a.fx, a.g, a.write_moments != 0, mom);
+        const bool enter = a.fx.ok && fixed_range(fv);
+        if (enter) {
+            let_next_start();
+            good = collide_fixed<PH::regularized>(fv, a.fx, a.g, a.write_moments != 0, mom);
+        }
         if (!good) {
-            // outside the fixed-point range: the site is read again and takes
-            // the FP64 form
-            C g[Q];
-            gather(g);
-            PH::collide_cold(g, a.g, a.w_e, a.w_o, mom);
-            Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
+            // outside the fixed-point range: the same
+            if constexpr (PH::fallback_inline) {
+                if (enter) gather(fv);
+                mom[0] = PH::collide(fv, a.g[0], a.g[1], a.g[2], a.w_e, a.w_o, mom[1], mom[2], mom[3]);
+            } else {
+                C g[Q];
+                if (enter) gather(g);
+                else Unroll<0, Q>::run([&]<int q>() { g[q] = fv[q]; });
+                PH::collide_cold(g, a.g, a.w_e, a.w_o, mom);
+                Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
+            }
         }
         rho = mom[0]; ux = mom[1]; uy = mom[2]; uz = mom[3];
     } else {
