@@ -173,10 +173,8 @@ int launch_batch_step(const BatchArgs &a, int scheme, bool pstep, int block, int
 // rates, body force and face kinds of each node's domain.
 template <int SCH, bool PSTEP>
 __global__ void __launch_bounds__(128) lbm_batch_special_kernel(const BatchArgs a) {
-    // whole blocks of the tables: the first may begin before the launch's nodes
-    const int b = a.sp0 / (int)blockDim.x + (int)blockIdx.x;
-    const int t = b * (int)blockDim.x + (int)threadIdx.x;
-    if (t < a.sp0 || t >= a.sp1) return;
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= a.Msp) return;
     const BatchDomain &D = a.dom[__ldg(a.sp_dom + t)];
     StepArgs s{};
     s.f = a.f;
@@ -200,12 +198,12 @@ __global__ void __launch_bounds__(128) lbm_batch_special_kernel(const BatchArgs 
         s.gf[c] = D.g[c];
     }
     for (int f = 0; f < 6; ++f) s.bc[f] = D.bc[f];
-    special_node<StoreF32, PhysSh<SCH>, PSTEP, false>(s, b);
+    special_node<StoreF32, PhysSh<SCH>, PSTEP, false>(s, (int)blockIdx.x);
 }
 
 int launch_batch_special(const BatchArgs &a, int scheme, bool pstep, cudaStream_t st) {
-    if (a.sp1 <= a.sp0) return 0;
-    const unsigned blocks = (unsigned)((a.sp1 + 127) / 128 - a.sp0 / 128);
+    if (a.Msp <= 0) return 0;
+    const unsigned blocks = (unsigned)((a.Msp + 127) / 128);
 #define JLB_BS2(SCH) \
     if (pstep) lbm_batch_special_kernel<SCH, true><<<blocks, 128, 0, st>>>(a); \
     else lbm_batch_special_kernel<SCH, false><<<blocks, 128, 0, st>>>(a);

@@ -46,7 +46,6 @@ struct BatchArgs {
     // single-domain table layout ([19][Msp] element indices into f, Zou-He
     // data fixed at set-up) with the domain of each
     int Msp;
-    int sp0, sp1;          // boundary nodes [sp0, sp1) of the launch
     const int32_t *sp_dom;
     const int64_t *sp_node, *sp_rd, *sp_wr;
     const uint32_t *sp_info;

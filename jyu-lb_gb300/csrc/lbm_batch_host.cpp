@@ -21,6 +21,13 @@
 using namespace jlb;
 using namespace jlb_host;
 
+// positions [first, last) of jlb_batch::order
+struct BatchGroup {
+    int first, last;
+    bool special;  // its domains hold boundary nodes: all of the ensemble's
+    bool resident; // its populations stay in the L2 from step to step
+};
+
 struct jlb_batch {
     int scheme = 0;
     int ndom = 0;
@@ -42,9 +49,10 @@ struct jlb_batch {
     double tune_ms[3] = {0, 0, 0}; // per-step time of blocks 64 / 128 / 256
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
     int GK = 32;
-    // runs of domains [first, last) advanced one after another, each for all
-    // steps of a call; group_bytes bounds their populations
-    std::vector<std::pair<int, int>> groups;
+    // domains in the order of their tiles, and the runs of it that are advanced
+    // one after another, each for all steps of a call (batch_groups)
+    std::vector<int> order;
+    std::vector<BatchGroup> groups;
     double group_bytes = 0;
     // boundary nodes of domains with Zou-He or symmetric faces (device
     // tables in the single-domain layout, element indices into f)
@@ -101,8 +109,6 @@ BatchArgs batch_args(const jlb_batch *b, int write_moments) {
     a.write_moments = write_moments;
     a.tile0 = 0;
     a.ntiles = b->ntiles;
-    a.sp0 = 0;
-    a.sp1 = b->Msp;
     a.pf = b->pf;
     a.Msp = b->Msp;
     a.sp_dom = b->d_sp_dom;
@@ -116,7 +122,7 @@ BatchArgs batch_args(const jlb_batch *b, int write_moments) {
 // tile table for block size `block`; also sets first_tile of every domain
 int batch_tiles(jlb_batch *b, int block) {
     std::vector<int32_t> td;
-    for (int d = 0; d < b->ndom; ++d) {
+    for (int d : b->order) {
         b->dom[d].first_tile = (int32_t)td.size();
         const int nt = (b->dom[d].n + block - 1) / block;
         for (int t = 0; t < nt; ++t) td.push_back(d);
@@ -144,22 +150,90 @@ int batch_tiles(jlb_batch *b, int block) {
     return JLB_OK;
 }
 
-// one step of the domains [d0, d1)
-int batch_launch(jlb_batch *b, bool pstep, int write_moments, int d0, int d1) {
+// Groups of domains whose populations stay in the L2 (129 MB) from step to step.
+// Domains do not touch each other, so a group may run all steps of a call before
+// the next one begins.  us a step in long calls, together / in groups: 32
+// channels (1.8 GB) 555 / 485, 3 channels (173 MB) 52.6 / 45.9; 32 channels (0.9
+// GB) in groups of 30 / 45 / 64 / 80 / 100 MB 229.6 / 215.8 / 212.2 / 209.2 /
+// 209.8 against 245.9.  group_bytes is 0.65 of the L2 (84 MB).
+//   * An ensemble of up to 1.25 of it stays together (3 x 30 MB 21.7 / 22.7).
+//   * Domains with boundary nodes run together: their second launch a step does
+//     not overlap the first (32 ducts, 1.8 GB: 615 / 779).
+//   * A larger domain is a group by itself (8 x 150 MB 358 / 339, 2 x 800 MB 483
+//     / 481).
+//   * The others fill groups evenly, whatever their place in the list.  What is
+//     left below a quarter joins the group before it (112 MB and 0.2 MB 29.8 /
+//     32.2, and 10 MB 32.9 / 33.9, and 20 MB 36.3 / 36.0, and 40 MB 44.0 / 40.9).
+void batch_groups(jlb_batch *b) {
+    const double cap = b->group_bytes;
+    auto bytes = [&](int d) { return 19.0 * sizeof(float) * b->dom[d].n; };
+    std::vector<int> special, large, small;
+    double total = 0, rest = 0;
+    for (int d = 0; d < b->ndom; ++d) {
+        total += bytes(d);
+        if (b->sp_first[d + 1] > b->sp_first[d]) special.push_back(d);
+        else if (bytes(d) > cap) large.push_back(d);
+        else { small.push_back(d); rest += bytes(d); }
+    }
+    b->order.clear();
+    b->groups.clear();
+    if (cap <= 0 || total <= 1.25 * cap) {
+        for (int d = 0; d < b->ndom; ++d) b->order.push_back(d);
+        b->groups.push_back({0, b->ndom, b->Msp > 0, false});
+        return;
+    }
+    auto append = [&](const std::vector<int> &v) { b->order.insert(b->order.end(), v.begin(), v.end()); };
+    append(special);
+    if (!special.empty()) b->groups.push_back({0, (int)special.size(), true, false});
+    append(large);
+    for (int i = 0; i < (int)large.size(); ++i) {
+        const int at = (int)special.size() + i;
+        b->groups.push_back({at, at + 1, false, false});
+    }
+    // consecutive small domains up to `limit` bytes a group; sizes of the groups
+    auto fill = [&](double limit, std::vector<std::pair<int, double>> &out) {
+        out.clear();
+        for (int d : small) {
+            if (out.empty() || out.back().second + bytes(d) > limit) out.push_back({0, 0.0});
+            ++out.back().first;
+            out.back().second += bytes(d);
+        }
+    };
+    std::vector<std::pair<int, double>> runs, even;
+    fill(cap, runs);
+    // the least limit that needs no more groups, to 2%
+    if (runs.size() > 1)
+        for (double limit = rest / (double)runs.size(); limit < cap; limit *= 1.02) {
+            fill(limit, even);
+            if (even.size() <= runs.size()) { runs = even; break; }
+        }
+    append(small);
+    int at = (int)(special.size() + large.size());
+    for (size_t i = 0; i < runs.size(); ++i) {
+        const int last = at + runs[i].first;
+        const bool alone = i > 0 && runs[i - 1].second + runs[i].second > 1.25 * cap;
+        if (i + 1 == runs.size() && runs[i].second < 0.25 * cap && !b->groups.empty() && !alone)
+            b->groups.back().last = last;
+        else
+            b->groups.push_back({at, last, false, true});
+        at = last;
+    }
+}
+
+// one step of the tiles of a group
+int batch_launch(jlb_batch *b, bool pstep, int write_moments, const BatchGroup &g) {
     BatchArgs a = batch_args(b, write_moments);
-    a.tile0 = b->dom[d0].first_tile;
-    a.ntiles = (d1 < b->ndom ? b->dom[d1].first_tile : b->ntiles) - a.tile0;
-    a.sp0 = b->sp_first.empty() ? 0 : b->sp_first[d0];
-    a.sp1 = b->sp_first.empty() ? 0 : b->sp_first[d1];
-    // a group that stays in the L2 needs no prefetch into it
-    if (b->groups.size() > 1 && 76.0 * (double)a.ntiles * b->block <= b->group_bytes + 76.0 * 128 * (d1 - d0)) a.pf = 0;
+    a.tile0 = b->dom[b->order[g.first]].first_tile;
+    a.ntiles = (g.last < b->ndom ? b->dom[b->order[g.last]].first_tile : b->ntiles) - a.tile0;
+    if (!g.special) a.Msp = 0;
+    if (g.resident) a.pf = 0; // no prefetch into what the L2 holds
     // from the end where the last step left its lines in the L2: 32 channels
     // (0.9 GB) 254.7 -> 248.2 us a step
     a.rev = !pstep;
     int r = launch_batch_step(a, b->scheme, pstep, b->block, a.ntiles, b->st);
     if (r) return bfail(b, JLB_ERR_CUDA, std::string("batch step: ") + cudaGetErrorString((cudaError_t)r));
     ++b->launches;
-    if (a.sp1 > a.sp0) {
+    if (a.Msp > 0) {
         r = launch_batch_special(a, b->scheme, pstep, b->st);
         if (r) return bfail(b, JLB_ERR_CUDA, std::string("batch boundary nodes: ") + cudaGetErrorString((cudaError_t)r));
         ++b->launches;
@@ -167,12 +241,24 @@ int batch_launch(jlb_batch *b, bool pstep, int write_moments, int d0, int d1) {
     return JLB_OK;
 }
 
+// all domains in one launch (and one for the boundary nodes)
+int batch_launch(jlb_batch *b, bool pstep, int write_moments) {
+    return batch_launch(b, pstep, write_moments, BatchGroup{0, b->ndom, b->Msp > 0, false});
+}
+
+// Calls of fewer steps run all domains together: a group's first step finds
+// nothing in the L2, and its launch ends in a partial wave.  us a step together /
+// in groups at 1, 2, 3, 4 steps a call: 512 channels (29 GB) 9337 / 11033, 10361 /
+// 10721, 9709 / 9781, 10130 / 9903; 32 channels 580 / 688, 589 / 597, 563 / 553,
+// 571 / 541; 8 x 150 MB 385 / 413, 381 / 382, 368 / 365, 370 / 360
+constexpr uint32_t GROUP_STEPS = 4;
+
 int batch_run(jlb_batch *b, uint32_t n, bool write_last) {
     uint32_t plain = write_last && n > 0 ? n - 1 : n;
-    if (b->groups.size() > 1) {
-        for (const auto &g : b->groups)
+    if (b->groups.size() > 1 && n >= GROUP_STEPS) {
+        for (const BatchGroup &g : b->groups)
             for (uint32_t t = 0; t < n; ++t) {
-                int r = batch_launch(b, ((b->parity + t) & 1) == 0, write_last && t + 1 == n, g.first, g.second);
+                int r = batch_launch(b, ((b->parity + t) & 1) == 0, write_last && t + 1 == n, g);
                 if (r) return r;
             }
         b->parity ^= (int)(n & 1);
@@ -185,7 +271,7 @@ int batch_run(jlb_batch *b, uint32_t n, bool write_last) {
             BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
             int par = p, rr = JLB_OK;
             for (int t = 0; t < b->GK && rr == JLB_OK; ++t) {
-                rr = batch_launch(b, par == 0, 0, 0, b->ndom);
+                rr = batch_launch(b, par == 0, 0);
                 par ^= 1;
             }
             cudaError_t ce = cudaStreamEndCapture(b->st, &g);
@@ -202,12 +288,12 @@ int batch_run(jlb_batch *b, uint32_t n, bool write_last) {
         if (b->GK & 1) b->parity ^= 1;
     }
     for (uint32_t t = 0; t < plain; ++t) {
-        int r = batch_launch(b, b->parity == 0, 0, 0, b->ndom);
+        int r = batch_launch(b, b->parity == 0, 0);
         if (r) return r;
         b->parity ^= 1;
     }
     if (write_last && n > 0) {
-        int r = batch_launch(b, b->parity == 0, 1, 0, b->ndom);
+        int r = batch_launch(b, b->parity == 0, 1);
         if (r) return r;
         b->parity ^= 1;
     }
@@ -238,9 +324,9 @@ int batch_autotune(jlb_batch *b) {
     for (int c = 0; c < 3; ++c) {
         int r = batch_tiles(b, cand[c]);
         if (r) return r;
-        for (int t = 0; t < 2; ++t) if ((r = batch_launch(b, t == 0, 0, 0, b->ndom))) return r;
+        for (int t = 0; t < 2; ++t) if ((r = batch_launch(b, t == 0, 0))) return r;
         cudaEventRecord(e0, b->st);
-        for (int t = 0; t < 4; ++t) if ((r = batch_launch(b, t % 2 == 0, 0, 0, b->ndom))) return r;
+        for (int t = 0; t < 4; ++t) if ((r = batch_launch(b, t % 2 == 0, 0))) return r;
         cudaEventRecord(e1, b->st);
         cudaEventSynchronize(e1);
         float ms = 0;
@@ -548,29 +634,14 @@ int jlb_batch_create(int32_t scheme, const jlb_domain *doms, int32_t ndom, void 
         const char *e = std::getenv("JLB_BATCH_PF");
         if (e && e[0]) b->pf_tiles = std::max(0, std::atoi(e));
         const char *eg = std::getenv("JLB_BATCH_GROUP");
+        // JLB_BATCH_GROUP=<MB> sets the size, 0 keeps all domains together
         b->group_bytes = eg && eg[0] ? 1e6 * std::atof(eg) : 0.65 * (double)l2;
     }
+    batch_groups(b);
     const char *tune = std::getenv("JLB_BATCH_BLOCK");
     if (tune && tune[0]) r = batch_tiles(b, std::atoi(tune));
     else r = batch_autotune(b);
     if (r) return bail(r);
-    // Groups of consecutive domains whose populations stay in the L2 (129 MB)
-    // from step to step.  Domains do not touch each other, so a group may run
-    // all steps of a call before the next one begins; domains larger than that
-    // are groups by themselves.  32 channels (0.9 GB), us a step: all together
-    // 245.9, groups of 30 / 45 / 64 / 80 / 100 MB 229.6 / 215.8 / 212.2 / 209.2 /
-    // 209.8; 8 channels (76 MB): together 19.6, groups of 45 / 64 / 80 MB 23.0 /
-    // 21.2 / 19.6.  JLB_BATCH_GROUP=<MB> sets the size, 0 keeps them together.
-    double bytes = 0;
-    for (int d = 0; d < ndom; ++d) {
-        const double x = 19.0 * sizeof(float) * b->dom[d].n;
-        if (b->groups.empty() || (b->group_bytes > 0 && bytes + x > b->group_bytes)) {
-            b->groups.emplace_back(d, d);
-            bytes = 0;
-        }
-        b->groups.back().second = d + 1;
-        bytes += x;
-    }
     *out = b;
     return JLB_OK;
 }
