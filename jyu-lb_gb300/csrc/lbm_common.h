@@ -117,7 +117,14 @@ struct Consts64 {
 struct Force64 {
     double a[3], c1a[3], c2a[3];
     unsigned mask;
+    int plain; // 1: with these rates or this force, only the reference's own order of operations is safe
 };
+// x is zero or 2^lo <= |x| < 2^hi
+__host__ __device__ __forceinline__ bool zero_or_within(double x, int lo, int hi) {
+    const uint64_t u = soft64::bits(x);
+    const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+    return (u << 1) == 0 || e - (uint32_t)(1023 + lo) < (uint32_t)(hi - lo);
+}
 
 struct StepArgs {
     void *f;              // populations, 19 * Np elements of the storage type
@@ -215,6 +222,9 @@ inline void set_consts64(StepArgs &a, int scheme) {
         a.g64.c2a[d] = 2.0 * k.c2 * a.g[d];
         if (a.g[d] != 0.0) a.g64.mask |= 1u << d;
     }
+    // bounds that Phys64::ordinary() counts on
+    a.g64.plain = !(k.we > 0x1p-100 && k.we < 0x1p10 && k.wodd > 0x1p-100 && k.wodd < 0x1p10);
+    for (int d = 0; d < 3; ++d) a.g64.plain |= !zero_or_within(a.g[d], -400, 200);
 }
 
 // Blocks of the boundary-node path in a launch of the direct step kernel (or

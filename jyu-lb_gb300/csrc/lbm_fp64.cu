@@ -24,7 +24,8 @@ namespace jlb {
 //     and differences of the projection's even and odd parts on the integer
 //     pipes, beside the FP64 pipe: of about 210 FP64 operations of a TRT site
 //     77 are left, and both kinds of pipe take about as long.
-// Same bits as the plain form.  128^3 cavity, us a step: plain; with integer
+// Same bits as the plain form (collide_plain, which sites near overflow or
+// underflow take).  128^3 cavity, us a step: plain; with integer
 // moments and relaxation; with the reciprocal too; with the moments' and the
 // projection's constants; with its sums: TRT 1111, 562, 548, 490, 452; BGK 938,
 // 497, 479, 425, 383; regularized 938, 521, 502, 402, 366.
@@ -115,46 +116,116 @@ template <int SCH> struct Phys64 : Phys64Base {
         force(h, F, k, den, jx, jy, jz);
     }
 
+    // The update in the reference's own operations (jyulb/D3Q19.pyx:655-940).
+    // project_fused halves and doubles where the reference multiplies, and skips
+    // terms of zero force, which is the same until a number overflows, becomes
+    // denormal, or is not finite; ordinary() tells.
+    __device__ __noinline__ static C collide_plain(C *f, const Force64 &F, const Consts64 &k, C *u) {
+        const C ax = F.a[0], ay = F.a[1], az = F.a[2], we = k.we, wo = k.wodd;
+        C h[10];
+        if (SCH != SCH_REG) {
+            const C c2 = 1.0 - 0.5 * we, c1 = SCH == SCH_TRT ? 1.0 - 0.5 * wo : c2;
+            const C den = f_to_den_vel(f, u[0], u[1], u[2]);
+            u[0] = u[0] + 0.5 * ax; u[1] = u[1] + 0.5 * ay; u[2] = u[2] + 0.5 * az;
+            heq(den, u[0], u[1], u[2], h);
+#pragma unroll
+            for (int m = 0; m < 10; ++m) h[m] = h[m] * (m >= 1 && m <= 3 ? wo : we);
+            const C jx = den * u[0], jy = den * u[1], jz = den * u[2];
+            h[1] = h[1] + c1 * ax * den; h[2] = h[2] + c1 * ay * den; h[3] = h[3] + c1 * az * den;
+            force_h2(h, c2, ax, ay, az, jx, jy, jz);
+            relax(f, k);
+            project<true>(h, f);
+            return den;
+        } else {
+            const C c2 = 1.0 - 0.5 * we;
+            C he[10];
+            f_to_h(f, h);
+            const C den = h[0], inv = 1.0 / den;
+            const C jx = h[1] + 0.5 * ax * den, jy = h[2] + 0.5 * ay * den, jz = h[3] + 0.5 * az * den;
+            u[0] = inv * jx; u[1] = inv * jy; u[2] = inv * jz;
+            heq(den, u[0], u[1], u[2], he);
+#pragma unroll
+            for (int m = 0; m < 10; ++m) h[m] = h[m] * k.r9 + we * he[m];
+            h[1] = h[1] + c2 * ax * den; h[2] = h[2] + c2 * ay * den; h[3] = h[3] + c2 * az * den;
+            force_h2(h, c2, ax, ay, az, jx, jy, jz);
+            project<false>(h, f);
+            return den;
+        }
+    }
+    // density in [2^-100, 2^100) and velocity components that are zero or in
+    // [2^-200, 2^200) (regularized: momenta and second moments): with the bounds
+    // of Force64::plain every product and sum of the update is then zero or in
+    // [2^-900, 2^1000)
+    template <int N> __device__ static bool ordinary(C den, const C *x) {
+        const uint32_t e = (uint32_t)(soft64::bits(den) >> 52) & 0x7ffu;
+        bool ok = e - (1023u - 100u) < 200u;
+#pragma unroll
+        for (int i = 0; i < N; ++i) ok = ok && zero_or_within(x[i], -200, 200);
+        return ok;
+    }
+    __device__ static C plain_site(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz) {
+        C g[Q], u[3]; // collide_plain takes addresses
+#pragma unroll
+        for (int q = 0; q < Q; ++q) g[q] = f[q];
+        const C den = collide_plain(g, F, k, u);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) f[q] = g[q];
+        ux = u[0]; uy = u[1]; uz = u[2];
+        return den;
+    }
+
+    // f_q <- c3 f_q - c4 f_opp (BGK: (1 - we) f_q)
+    __device__ static void relax(C *f, const Consts64 &k) {
+        if (SCH == SCH_BGK) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) f[q] = f[q] * k.r9;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                const C fa = f[q], fb = f[18 - q];
+                f[q] = k.c3 * fa - k.c4 * fb;
+                f[18 - q] = k.c3 * fb - k.c4 * fa;
+            }
+            f[9] = f[9] * k.r9;
+        }
+    }
+    // moments of f (jyulb/D3Q19.pyx:395-452)
+    __device__ static void f_to_h(const C *f, C *h) {
+        C d1x = f[0] + f[1] + f[2] + f[3] + f[4];
+        C dx1 = f[14] + f[15] + f[16] + f[17] + f[18];
+        C d01y = f[5] + f[6] + f[7];
+        C d0y1 = f[11] + f[12] + f[13];
+        C d1y = f[0] + d01y + f[14];
+        C dy1 = f[4] + d0y1 + f[18];
+        C d1z = f[1] + f[5] + f[8] + f[11] + f[15];
+        C dz1 = f[3] + f[7] + f[10] + f[13] + f[17];
+        C den = d1x + dx1 + d01y + d0y1 + f[8] + f[9] + f[10];
+        h[0] = den; h[1] = dx1 - d1x; h[2] = dy1 - d1y; h[3] = dz1 - d1z;
+        const C d3 = (1.0 / 3.0) * den;
+        h[4] = (d1x + dx1) - d3;
+        h[5] = f[0] + f[18] - f[4] - f[14];
+        h[6] = f[1] + f[17] - f[3] - f[15];
+        h[7] = (d1y + dy1) - d3;
+        h[8] = f[5] + f[13] - f[7] - f[11];
+        h[9] = (d1z + dz1) - d3;
+    }
+
     // forward-Euler update; returns den, writes the stored velocity
     // u = j/den + a/2 (jyulb/D3Q19.pyx:655-940)
     __device__ static C collide(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz) {
         C h[10];
         if (SCH != SCH_REG) {
             const C den = f_to_den_vel(f, ux, uy, uz);
+            const C u[3] = {ux, uy, uz};
+            if (F.plain || !ordinary<3>(den, u)) return plain_site(f, F, k, ux, uy, uz);
             relaxed_moments<false>(h, F, k, den, ux, uy, uz);
-            if (SCH == SCH_BGK) {
-#pragma unroll
-                for (int q = 0; q < Q; ++q) f[q] = f[q] * k.r9;
-            } else {
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    const C fa = f[q], fb = f[18 - q];
-                    f[q] = k.c3 * fa - k.c4 * fb;
-                    f[18 - q] = k.c3 * fb - k.c4 * fa;
-                }
-                f[9] = f[9] * k.r9;
-            }
+            relax(f, k);
             project_fused<true>(h, f);
             return den;
         } else {
-            // f_to_h (jyulb/D3Q19.pyx:395-452)
-            C d1x = f[0] + f[1] + f[2] + f[3] + f[4];
-            C dx1 = f[14] + f[15] + f[16] + f[17] + f[18];
-            C d01y = f[5] + f[6] + f[7];
-            C d0y1 = f[11] + f[12] + f[13];
-            C d1y = f[0] + d01y + f[14];
-            C dy1 = f[4] + d0y1 + f[18];
-            C d1z = f[1] + f[5] + f[8] + f[11] + f[15];
-            C dz1 = f[3] + f[7] + f[10] + f[13] + f[17];
-            C den = d1x + dx1 + d01y + d0y1 + f[8] + f[9] + f[10];
-            h[0] = den; h[1] = dx1 - d1x; h[2] = dy1 - d1y; h[3] = dz1 - d1z;
-            const C d3 = (1.0 / 3.0) * den;
-            h[4] = (d1x + dx1) - d3;
-            h[5] = f[0] + f[18] - f[4] - f[14];
-            h[6] = f[1] + f[17] - f[3] - f[15];
-            h[7] = (d1y + dy1) - d3;
-            h[8] = f[5] + f[13] - f[7] - f[11];
-            h[9] = (d1z + dz1) - d3;
+            f_to_h(f, h);
+            if (F.plain || !ordinary<9>(h[0], h + 1)) return plain_site(f, F, k, ux, uy, uz);
+            const C den = h[0];
             relaxed_moments_reg<false>(h, F, k, 1.0 / h[0], ux, uy, uz);
             project_fused<false>(h, f);
             return den;

@@ -168,6 +168,7 @@ template <bool ACCF> __device__ __forceinline__ Force64 site_force64(const StepA
             F.a[d] = a.g[d] + __ldg(acc + d * a.Np + n);
             F.c1a[d] = a.c1 * F.a[d];
             F.c2a[d] = 2.0 * a.k64.c2 * F.a[d];
+            F.plain |= !zero_or_within(F.a[d], -400, 200);
         }
         F.mask = 7u;
     }

@@ -85,4 +85,42 @@ def test_cost_outside_the_ranges(fast, lat, rho, u):
             best = min(best, time.perf_counter() - t)
         return best
 
-    assert us(0.0) <= 1.08 * us(0.07 if fast else 1e-310)
+    assert us(0.0) <= 1.08 * us(0.07 if fast else 1e-100)
+
+
+# flows near overflow and underflow, bulk and lid sites: the parity form keeps
+# the reference's infinities, NaN and denormal roundings
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("bc", [[1, 1, 0, 0, 1, 1], [0, 0, 0, 3, 0, 0]])
+@pytest.mark.parametrize("g", [0.0, 2e-5, 1e-130])
+@pytest.mark.parametrize("kind,value", [("speed", v) for v in (1e145, 5e150, 2e151, 1e152, 5e152, 2e153, 1e154, 1e160)] +
+                         [("density", v) for v in (1e-308, 1e-306, 1e-304, 1e300, 3e307)] +
+                         [("site", v) for v in (3e152, 1e153, 1e154, 3e155)])
+def test_overflow_and_underflow(scheme, bc, g, kind, value):
+    from jyulb.defs import FP64
+    from jyulb.isothermal import Solver
+    from pyoracle import Oracle
+
+    lat = (5, 6, 12)
+    rng = np.random.default_rng(24)
+    den = 1 + 0.01 * rng.uniform(-1, 1, lat)
+    vel = 0.02 * rng.uniform(-1, 1, lat + (3,))
+    if kind == "speed":
+        vel *= 50 * value
+    elif kind == "density":
+        den *= value
+    else:
+        vel[2, 2, 5] = value
+    for steps in (1, 2, 3, 5):
+        s = Solver(np.array(lat, np.int32), scheme, 0.05, np.array([0, g, 0]), np.array(bc, np.int32), precision=FP64)
+        o = Oracle(lat, scheme, 0.05, (0, g, 0), bc, 0.0)
+        with np.errstate(all="ignore"):
+            for x in (s, o):
+                x.get_phase()[:] = 1
+                x.get_den()[:] = den
+                x.get_vel()[:] = vel
+                x.finalize_init()
+                x.evolve(steps)
+            assert np.array_equal(s.populations(), o.populations(), equal_nan=True)
+            assert np.array_equal(s.get_vel(), o.get_vel(), equal_nan=True)
+            assert np.array_equal(s.get_den(), o.get_den(), equal_nan=True)
