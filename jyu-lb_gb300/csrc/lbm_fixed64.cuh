@@ -70,22 +70,14 @@ inline FixConsts make_fix_consts(bool trt, bool reg, double we, double wo, const
     return k;
 }
 
-// populations of the form's range: in [2^-9, 1/8), the rest one in [1/8, 1/2).
-// Looked at before anything else, so that a site outside (a density not near 1)
-// pays for nothing but the FP64 form.
-S64_FN bool fixed_range(const double *f) {
-    uint32_t range = 0;
-#pragma unroll
-    for (int q = 0; q < 19; ++q) {
-        const uint32_t r = soft64::fix_range(f[q]);
-        if (q != 9) range = range > r ? range : r;
-    }
-    return range < (6u << 20) && soft64::fix_range(f[9]) - (6u << 20) < (2u << 20);
-}
+// What the density's range leaves the rest population, near equilibrium.  Looked
+// at before anything else, so that a site with a density not near 1 pays for
+// nothing but the FP64 form.
+S64_FN bool fixed_range(const double *f) { return soft64::within(f[9], 0.125, 0.5); }
 
 // f[19] in place; returns false where an operand leaves the form's range:
-// populations in fixed_range() before and at least 2^-9 after, density in
-// [1/2 + 2^-29, 3/2), |j + a den/2| < 1/4 per component; f is then undefined.
+// populations in [2^-9, 1/8) (rest: fixed_range()) before and at least 2^-9
+// after, density in [1/2 + 2^-29, 3/2), |j + a den/2| < 1/4 per component; f is then undefined.
 // (From density 1/2 itself the reciprocal, with unit 2^-62, would reach 2^63: the
 // margin leaves digits() the 2^31 it adds.)  With `want`, mom receives den and
 // the stored velocity u = j/den + a/2.
@@ -93,9 +85,10 @@ template <bool REG>
 S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool want, double *mom) {
     using namespace soft64;
     if (!fixed_range(f)) return false;
+    uint32_t range = 0, rest = 0;
     int64_t x[19];
 #pragma unroll
-    for (int q = 0; q < 19; ++q) x[q] = (int64_t)fix(f[q]);
+    for (int q = 0; q < 19; ++q) x[q] = (int64_t)fix(f[q], q == 9 ? rest : range);
     // even and odd parts of the pairs, by the index of their p: 10 (0,0,1),
     // 11 (0,1,-1), 12 (0,1,0), 13 (0,1,1), 14 (1,-1,0), 15 (1,0,-1),
     // 16 (1,0,0), 17 (1,0,1), 18 (1,1,0)
@@ -125,7 +118,8 @@ S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool w
         u[d] = mulq(s[d] * 8, iv);
         sd[d] = digits(s[d]);
     }
-    if (fast >= (1u << 28) || (uint32_t)((uint64_t)den >> 32) - ((1u << 28) + 1u) >= (1u << 29) - 1u) return false;
+    if (range > 5u || fast >= (1u << 28) || (uint32_t)((uint64_t)den >> 32) - ((1u << 28) + 1u) >= (1u << 29) - 1u)
+        return false;
     if (want) {
         mom[0] = dd;
 #pragma unroll

@@ -231,39 +231,30 @@ template <int SCH> struct Phys64 : Phys64Base {
             return den;
         }
     }
-    // the FP64 form of a site that collide_int refuses: out of line (128^3, us a
-    // step of accepted sites, inline / out of line: BGK 375 / 362, TRT 450 / 433,
-    // regularized 350 / 358)
-    static constexpr bool fallback_inline = SCH == SCH_REG;
+    // the FP64 form of a site that collide_int refuses, out of line: inline, the
+    // accepted sites lose (128^3, us a step: BGK 362 -> 375, TRT 433 -> 450)
     __device__ __noinline__ static C collide_cold(C *f, const Force64 &F, const Consts64 &k, C *u) {
         return collide(f, F, k, u[0], u[1], u[2]);
     }
 
-    // populations of collide_int's range: in [2^-9, 1/4), the rest one below 2
-    // (the sum then stays below 2^64 units).  Looked at before anything else, so
-    // that a site outside pays for nothing but the FP64 form.
-    __device__ static bool int_range(const C *f) {
-        uint32_t range = 0;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const uint32_t r = soft64::fix_range(f[q]);
-            if (q != 9) range = range > r ? range : r;
-        }
-        return range < (7u << 20) && soft64::fix_range(f[9]) < (10u << 20);
-    }
+    // What collide_int's range leaves the rest population, near equilibrium.
+    // Looked at before anything else, so that a site with a density far from 1
+    // pays for nothing but the FP64 form.
+    __device__ static bool int_range(const C *f) { return soft64::within(f[9], 0x1p-5, 1.5); }
 
     // The same update, with most of its operations on the integer pipes
-    // (soft64.cuh): the same bits.  It needs populations in int_range(),
-    // velocities that are zero or in [2^-400, 2^8), and projections whose even
-    // parts outweigh the odd ones; anything else sets `bad` and leaves f undefined.
+    // (soft64.cuh): the same bits.  It needs populations in [2^-9, 1/4) (rest:
+    // int_range(); the sum then stays below 2^64 units), velocities that are zero
+    // or in [2^-400, 2^8), and projections whose even parts outweigh the odd ones;
+    // anything else sets `bad` and leaves f undefined.
     __device__ static C collide_int(C *f, const Force64 &F, const Consts64 &k, C &ux, C &uy, C &uz, bool &bad) {
         using namespace soft64;
         C h[10], den, inv;
-        uint32_t least = 0;
+        uint32_t range = 0, rest = 0, least = 0;
         {
             uint64_t x[Q];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) x[q] = fix(f[q]);
+            for (int q = 0; q < Q; ++q) x[q] = fix(f[q], q == 9 ? rest : range);
             const uint64_t d1x = add(add(add(add(x[0], x[1]), x[2]), x[3]), x[4]);
             const uint64_t dx1 = add(add(add(add(x[14], x[15]), x[16]), x[17]), x[18]);
             const uint64_t d01y = add(add(x[5], x[6]), x[7]);
@@ -337,8 +328,8 @@ template <int SCH> struct Phys64 : Phys64Base {
             relaxed_moments_reg<true>(h, F, k, inv, ux, uy, uz);
         }
         uint32_t span = 0;
-        int32_t apart = 1 << 30;
-        project_int<SCH != SCH_REG>(h, k, f, span, apart, least);
+        int32_t apart = 1 << 30, close = 1 << 30;
+        project_int<SCH != SCH_REG>(h, k, f, span, apart, close);
         // velocities are zero or in [2^-400, 2^8): their products, and those
         // with the force they bound, are normal.  An acceleration field may hold
         // anything; mul() of a NaN or an infinity would be some finite number
@@ -350,17 +341,18 @@ template <int SCH> struct Phys64 : Phys64Base {
             const uint32_t z = (u << 1) ? e - (1023u - 400u) : 0u;
             beyond = beyond > z ? beyond : z;
         }
-        bad = least >= (1u << 31) - (1u << 21) || span > PROJ_SPAN || apart < 0 || beyond > 407u;
+        bad = range > 6u || least >= (1u << 31) - (1u << 21) || span > PROJ_SPAN || apart < 0 || close < 1 << 21 ||
+              beyond > 407u;
         return den;
     }
 
     // project_fused with integer products and sums; `span` exceeds PROJ_SPAN
-    // unless every even part lies in [2^-40, 2^10); `apart` is negative or `least`
-    // 2^31 - 2^21 or more where an odd part is not smaller than its even one, or
-    // reaches it but for 2^-8 of the even one's binade
+    // unless every even part lies in [2^-40, 2^10); `apart` is negative or `close`
+    // below 2^21 where an odd part is not smaller than its even one, or reaches it
+    // but for 2^-8 of the even one's binade
     static constexpr uint32_t PROJ_LO = (1023u - 40u) << 20, PROJ_SPAN = (50u << 20) - 1u;
     template <bool ADD>
-    __device__ static void project_int(const C *h, const Consts64 &k, C *f, uint32_t &span, int32_t &apart, uint32_t &least) {
+    __device__ static void project_int(const C *h, const Consts64 &k, C *f, uint32_t &span, int32_t &apart, int32_t &close) {
         const C t4 = soft64::mulz(h[4], k.m3), t7 = soft64::mulz(h[7], k.m3), t9 = soft64::mulz(h[9], k.m3);
         const C s = h[0] + t4, v = __fma_rn(2.0, h[0], -t4);
         const C w = __fma_rn(2.0, s, -t7), v2 = __fma_rn(2.0, t7, v);
@@ -372,7 +364,7 @@ template <int SCH> struct Phys64 : Phys64Base {
             const uint32_t x = (uint32_t)__double2hiint(e) - PROJ_LO;
             span = span > x ? span : x;
             C plus, minus;
-            soft64::add_sub(e, o, plus, minus, apart, &least);
+            soft64::add_sub(e, o, plus, minus, apart, &close);
             put(lo, soft64::mul(minus, m));
             put(18 - lo, soft64::mul(plus, m));
         };

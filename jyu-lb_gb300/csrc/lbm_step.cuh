@@ -323,17 +323,12 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
         if (bad) {
             // outside the integer form's range: the site takes the FP64 form;
             // nothing is stored yet, so what was overwritten is read again
-            if constexpr (PH::fallback_inline) {
-                if (enter) gather(fv);
-                rho = PH::collide(fv, F, a.k64, ux, uy, uz);
-            } else {
-                C g[Q], u[3];
-                if (enter) gather(g);
-                else Unroll<0, Q>::run([&]<int q>() { g[q] = fv[q]; });
-                rho = PH::collide_cold(g, F, a.k64, u);
-                ux = u[0]; uy = u[1]; uz = u[2];
-                Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
-            }
+            C g[Q], u[3];
+            if (enter) gather(g);
+            else Unroll<0, Q>::run([&]<int q>() { g[q] = fv[q]; });
+            rho = PH::collide_cold(g, F, a.k64, u);
+            ux = u[0]; uy = u[1]; uz = u[2];
+            Unroll<0, Q>::run([&]<int q>() { fv[q] = g[q]; });
         }
     } else if constexpr (uses_fixed_point<PH>::value && !ACCF) {
         C mom[4];

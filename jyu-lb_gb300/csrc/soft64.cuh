@@ -130,9 +130,9 @@ S64_FN double mulz(double x, const MulC &k) {
 // (which only a shift by 10 or more sets), added and subtracted, and both results
 // rounded, the smaller from at least 2^53 units of e's exponent - 61, that is
 // 2^-8 of e's binade.  `least` collects the exponent difference (negative for a
-// larger o); `p`, if given, what is 2^31 - 2^21 or more for a smaller or
-// negative difference.  |o| < e / 2 needs no such check.
-S64_FN void add_sub(double e, double o, double &plus, double &minus, int32_t &least, uint32_t *p = nullptr) {
+// larger o); `close`, if given, the high word of the aligned difference, below
+// 2^21 for a smaller or negative one.  |o| < e / 2 needs no such check.
+S64_FN void add_sub(double e, double o, double &plus, double &minus, int32_t &least, int32_t *close = nullptr) {
     const uint64_t ue = bits(e), uo = bits(o);
     const uint32_t eh = (uint32_t)(ue >> 32), oh = (uint32_t)(uo >> 32);
     const uint32_t oe = (oh >> 20) & 0x7ffu;
@@ -143,9 +143,9 @@ S64_FN void add_sub(double e, double o, double &plus, double &minus, int32_t &le
     const uint32_t sh = (uint32_t)r & 0x80000000u ? 0u : (uint32_t)r < 63u ? (uint32_t)r : 63u;
     const uint64_t v = mo >> sh;
     const uint64_t jam = v | ((v << sh) != mo ? 1u : 0u);
-    if (p) {
-        const uint32_t q = (uint32_t)((me - jam) >> 32) - (1u << 21);
-        *p = *p > q ? *p : q;
+    if (close) {
+        const int32_t q = (int32_t)(uint32_t)((me - jam) >> 32);
+        *close = *close < q ? *close : q;
     }
     auto round = [&](uint64_t s) { // [2^53, 2^63)
         const uint32_t hi = (uint32_t)(s >> 32), lo = (uint32_t)s;
@@ -166,23 +166,21 @@ S64_FN void add_sub(double e, double o, double &plus, double &minus, int32_t &le
 // ---------------------------------------------------------------------------
 constexpr uint32_t FIX_E0 = 1014; // exponent field of 2^-9, the least operand
 
-// x as fixed point, 2^-9 <= x < 2^2
-S64_FN uint64_t fix(double x) {
+// x in [2^-9, 2^(n-9)) as fixed point; `range` collects field - 1014, which is
+// n or more for anything else (negative numbers, zeros, infinities, NaN)
+S64_FN uint64_t fix(double x, uint32_t &range) {
     const uint64_t u = bits(x);
     const uint32_t xh = (uint32_t)(u >> 32), xl = (uint32_t)u;
-    const uint32_t s = ((xh >> 20) - FIX_E0) & 31u;
-    const uint32_t h = (xh & 0xfffffu) | 0x100000u;
-    return ((uint64_t)shl_hi(xl, h, s) << 32) | (uint32_t)(xl << s);
-}
-// x's distance from 2^-9 in high words: below n << 20 for x in [2^-9, 2^(n-9)),
-// n << 20 or more for anything else (negative numbers, zeros, infinities, NaN)
-S64_FN uint32_t fix_range(double x) { return (uint32_t)(bits(x) >> 32) - (FIX_E0 << 20); }
-// the same at once; `range` collects field - 1014, which is n or more for
-// anything else
-S64_FN uint64_t fix(double x, uint32_t &range) {
-    const uint32_t s = (uint32_t)(bits(x) >> 52) - FIX_E0;
+    const uint32_t s = (xh >> 20) - FIX_E0;
     range = range > s ? range : s;
-    return fix(x);
+    const uint32_t h = (xh & 0xfffffu) | 0x100000u;
+    return ((uint64_t)shl_hi(xl, h, s & 31u) << 32) | (uint32_t)(xl << (s & 31u));
+}
+// lo <= x < hi for positive bounds of at most 20 significant bits, by x's high
+// word (false for negative numbers and NaN)
+S64_FN bool within(double x, double lo, double hi) {
+    const uint32_t l = (uint32_t)(bits(lo) >> 32), h = (uint32_t)(bits(hi) >> 32);
+    return (uint32_t)(bits(x) >> 32) - l < h - l;
 }
 
 // a + b for positive operands (the sum is at least 2^53 units)

@@ -1,6 +1,6 @@
 """The integer forms of FP64 operations (csrc/soft64.cuh) over the operands the
 collision passes them: sums and differences of numbers close in size,
-reciprocals up to the largest density, and the range words."""
+reciprocals up to the largest density, and the check of a range."""
 import ctypes
 import os
 import shutil
@@ -15,24 +15,24 @@ SRC = r"""
 #include "soft64.cuh"
 using namespace jlb::soft64;
 extern "C" {
-void s_add_sub(const double *e, const double *o, double *p, double *m, int *least, unsigned *close, long n) {
+void s_add_sub(const double *e, const double *o, double *p, double *m, int *least, int *close, long n) {
     for (long i = 0; i < n; ++i) {
-        int32_t l = 1 << 30;
-        uint32_t c = 0;
+        int32_t l = 1 << 30, c = 1 << 30;
         add_sub(e[i], o[i], p[i], m[i], l, &c);
         least[i] = l;
         close[i] = c;
     }
 }
 void s_recip(const double *x, const double *y, double *s, double *o, long n) {
+    uint32_t range = 0;
     for (long i = 0; i < n; ++i) {
-        const uint64_t a = add(fix(x[i]), fix(y[i]));
+        const uint64_t a = add(fix(x[i], range), fix(y[i], range));
         s[i] = to_double(a);
         o[i] = recip(a);
     }
 }
-void s_range(const double *x, unsigned *r, long n) {
-    for (long i = 0; i < n; ++i) r[i] = fix_range(x[i]);
+void s_within(const double *x, double lo, double hi, int *r, long n) {
+    for (long i = 0; i < n; ++i) r[i] = within(x[i], lo, hi);
 }
 }
 """
@@ -60,9 +60,9 @@ def test_sums_and_differences_of_close_numbers(lib):
     o[:k] = e[:k]                                               # no difference
     o[k: 2 * k] = np.nextafter(e[k: 2 * k], 0)                  # the smallest
     o[2 * k: 3 * k] = -e[2 * k: 3 * k] * (1 - 2.0 ** -rng.integers(1, 12, k).astype(float))
-    p, m, least, close = np.empty(n), np.empty(n), np.empty(n, np.int32), np.empty(n, np.uint32)
+    p, m, least, close = np.empty(n), np.empty(n), np.empty(n, np.int32), np.empty(n, np.int32)
     lib.s_add_sub(ptr(e), ptr(o), ptr(p), ptr(m), ptr(least), ptr(close), ctypes.c_long(n))
-    fine = (least >= 0) & (close < (1 << 31) - (1 << 21))
+    fine = (least >= 0) & (close >= 1 << 21)
     binade = np.ldexp(1.0, np.frexp(e)[1] - 1)
     with np.errstate(over="ignore"):
         assert np.array_equal(fine, (np.frexp(o)[1] <= np.frexp(e)[1]) & (e - np.abs(o) >= binade * 2.0 ** -8))
@@ -76,16 +76,14 @@ def test_reciprocals_of_large_densities(lib):
     s, o = np.empty(n), np.empty(n)
     lib.s_recip(ptr(x), ptr(y), ptr(s), ptr(o), ctypes.c_long(n))
     assert same_bits(s, x + y) and same_bits(o, 1.0 / (x + y))
-    # nineteen populations: the sum of the largest that are accepted, 6.5
-    top = 18 * np.nextafter(0.25, 0) + np.nextafter(2, 0)
-    assert top < 8.0
+    # nineteen populations: the sum of the largest that are accepted
+    assert 18 * np.nextafter(0.25, 0) + 1.5 < 8.0
 
 
-@pytest.mark.parametrize("n", [6, 7, 10])
-def test_range_words(lib, n):
-    edge = 2.0 ** (n - 9)
-    x = np.array([2.0 ** -9, np.nextafter(edge, 0), 0.01, np.nextafter(2.0 ** -9, 0), edge, -0.01, -2.0 ** -9, 0.0, -0.0,
-                  5e-324, 1e300, np.inf, -np.inf, np.nan])
-    r = np.empty(len(x), np.uint32)
-    lib.s_range(ptr(x), ptr(r), ctypes.c_long(len(x)))
-    assert (r < (n << 20)).tolist() == [True] * 3 + [False] * 11
+@pytest.mark.parametrize("lo,hi", [(0.125, 0.5), (2.0 ** -5, 1.5), (2.0 ** -9, 0.25)])
+def test_within(lib, lo, hi):
+    x = np.array([lo, np.nextafter(hi, 0), 0.2, np.nextafter(lo, 0), hi, -0.2, -lo, 0.0, -0.0, 5e-324, 1e300, np.inf,
+                  -np.inf, np.nan])
+    r = np.empty(len(x), np.int32)
+    lib.s_within(ptr(x), ctypes.c_double(lo), ctypes.c_double(hi), ptr(r), ctypes.c_long(len(x)))
+    assert (r != 0).tolist() == [True] * 3 + [False] * 11
