@@ -81,7 +81,13 @@ S64_FN bool fixed_range(const double *f) { return soft64::within(f[9], 0.125, 0.
 // (From density 1/2 itself the reciprocal, with unit 2^-62, would reach 2^63: the
 // margin leaves digits() the 2^31 it adds.)  With `want`, mom receives den and
 // the stored velocity u = j/den + a/2.
-template <bool REG>
+//
+// The products that relax the even and odd parts round ties up, with DOWN down,
+// and the steps of the AA pair take turns.  A rate such as wo/12 = 1/16 (tau 0.8,
+// magic 1/4) makes a tie of every 16th product, and rounding all of them up
+// moved the momentum by 8e-19 a step and site, always the same way; FP64's own
+// bias is 1e-20 to 1e-19.
+template <bool REG, bool DOWN = false>
 S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool want, double *mom) {
     using namespace soft64;
     if (!fixed_range(f)) return false;
@@ -156,8 +162,8 @@ S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool w
         const int64_t base = 3 * (sxx + syy + szz) - (den >> 1);
         int64_t sum = 0;
         auto pair = [&](int i, int64_t y, int64_t b, int64_t odd) {
-            const int64_t E = mulq(9 * (fe[i] - y) + b, k.e);
-            const int64_t O = mulq(6 * fo[i] - odd, k.o);
+            const int64_t E = mulq<0, DOWN>(9 * (fe[i] - y) + b, k.e);
+            const int64_t O = mulq<0, DOWN>(6 * fo[i] - odd, k.o);
             sum += E;
             f[8 - i] = round_to_double(x[8 - i] - E + O, low);
             f[10 + i] = round_to_double(x[10 + i] - E - O, low);
@@ -188,7 +194,7 @@ S64_FN bool collide_fixed(double *f, const FixConsts &k, const double *a, bool w
         const int64_t base = ((den + 4) >> 3) - (xx + yy + zz); // 2 den - 3 tr H2
         int64_t sum = 0;
         auto pair = [&](int i, int64_t v, int64_t odd) {
-            const int64_t e = mulq(v, k.c72), o = mulq(odd, k.c12);
+            const int64_t e = mulq<0, DOWN>(v, k.c72), o = mulq<0, DOWN>(odd, k.c12);
             sum += e;
             f[8 - i] = round_to_double(e - o, low);
             f[10 + i] = round_to_double(e + o, low);

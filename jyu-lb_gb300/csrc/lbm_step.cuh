@@ -336,7 +336,7 @@ __device__ __forceinline__ void dense_node(const StepArgs &a, int b) {
         const bool enter = a.fx.ok && fixed_range(fv);
         if (enter) {
             let_next_start();
-            good = collide_fixed<PH::regularized>(fv, a.fx, a.g, a.write_moments != 0, mom);
+            good = collide_fixed<PH::regularized, !PSTEP>(fv, a.fx, a.g, a.write_moments != 0, mom);
         }
         if (!good) {
             // outside the fixed-point range: the same

@@ -286,12 +286,15 @@ S64_FN Fix2 digits(int64_t x) {
 // 2^63.  The collision's operands (lbm_fixed64.cuh), at most: 8 s 2^62 with the
 // reciprocal 2^63 - 2^34; momenta and velocities 2^61.2; 9 (fe - y) + b and
 // 6 fo - odd 2^62.6 with the rates 2^61.9; forces 2^60 with densities 2^61.6.
-template <int SH = 0> S64_FN int64_t mulq(const Fix2 &x, const Fix2 &y) {
-    int64_t m = (int64_t)x.lo * y.hi + (0x80000000ll >> SH);
+// Ties round up, with DOWN down.
+template <int SH = 0, bool DOWN = false> S64_FN int64_t mulq(const Fix2 &x, const Fix2 &y) {
+    int64_t m = (int64_t)x.lo * y.hi + ((0x80000000ll >> SH) - (DOWN ? 1 : 0));
     m = (int64_t)x.hi * y.lo + m;
     return (int64_t)x.hi * y.hi * (1ll << SH) + (m >> (32 - SH));
 }
-template <int SH = 0> S64_FN int64_t mulq(int64_t x, const Fix2 &y) { return mulq<SH>(digits(x), y); }
+template <int SH = 0, bool DOWN = false> S64_FN int64_t mulq(int64_t x, const Fix2 &y) {
+    return mulq<SH, DOWN>(digits(x), y);
+}
 
 // a positive number of 53 to 63 bits (unit 2^-61) rounded to a double;
 // `low` collects what makes it 2^31 - 2^20 or more for any other number
