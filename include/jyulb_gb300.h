@@ -234,8 +234,8 @@ typedef struct jlb_domain {
  * size with a timing autotuner (JLB_BATCH_BLOCK=64/128/256 fixes it). */
 int jlb_batch_create(int32_t rlx_scheme, const jlb_domain *doms, int32_t ndom, void *stream, jlb_batch **out);
 void jlb_batch_destroy(jlb_batch *b);
-/* advances every domain tsteps steps (one launch per step, graph-replayed);
- * moments of the last step are stored */
+/* advances every domain tsteps steps (one launch per step, graph-replayed, or
+ * per step and group of domains); moments of the last step are stored */
 int jlb_batch_step(jlb_batch *b, uint32_t tsteps);
 /* Zou-He data of domain d from den (nx,ny,nz) / vel (nx,ny,nz,3) at its
  * boundary sites, as Solver.evolve re-reads them at every call
@@ -245,7 +245,8 @@ int jlb_batch_step(jlb_batch *b, uint32_t tsteps);
  * moving solids), as Solver.evolve does.  Solid velocities stay as created.
  * Either pointer may be NULL (that field keeps its current values). */
 int jlb_batch_set_bc(jlb_batch *b, int32_t d, const double *den, const double *vel);
-/* den (nx,ny,nz) and vel (nx,ny,nz,3) of domain d on its fluid sites */
+/* den (nx,ny,nz) and vel (nx,ny,nz,3) of domain d on its fluid sites; threads
+ * may read different domains at once */
 int jlb_batch_moments(jlb_batch *b, int32_t d, double *den, double *vel);
 /* post-collision populations of domain d, (19, nx, ny, nz) FP64 */
 int jlb_batch_populations(jlb_batch *b, int32_t d, double *f);

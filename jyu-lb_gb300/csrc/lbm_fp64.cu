@@ -27,8 +27,9 @@ namespace jlb {
 // Same bits as the plain form (collide_plain, which sites near overflow or
 // underflow take).  128^3 cavity, us a step: plain; with integer
 // moments and relaxation; with the reciprocal too; with the moments' and the
-// projection's constants; with its sums: TRT 1111, 562, 548, 490, 452; BGK 938,
-// 497, 479, 425, 383; regularized 938, 521, 502, 402, 366.
+// projection's constants; with its sums; with the present range checks: TRT 1111,
+// 562, 548, 490, 452, 440; BGK 938, 497, 479, 425, 383, 378; regularized 938, 521,
+// 502, 402, 366, 366.
 template <int SCH> struct Phys64 : Phys64Base {
     static constexpr bool host_consts = true;
 

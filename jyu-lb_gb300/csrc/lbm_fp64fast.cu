@@ -6,8 +6,8 @@
 // (jyulb/D3Q19.pyx:655-940) with its forcing and stored velocity
 // u = j/den + a/2.  The bulk of the sites collides in 64-bit fixed point
 // (lbm_fixed64.cuh), which GB300's integer pipes do several times faster than
-// its FP64 pipe does FP64 and which loses less: 256^3 TRT cavity 5497 -> 1152
-// us a step, 128^3 699 -> 145, 40x33x27 15.2 -> 5.4.  Boundary nodes, sites
+// its FP64 pipe does FP64 and which loses less: 256^3 TRT cavity 5497 -> 1140
+// us a step, 128^3 699 -> 143, 40x33x27 15.2 -> 5.3.  Boundary nodes, sites
 // with an acceleration field and sites outside the fixed-point range take the
 // FP64 form below:
 //   * den, j and u in the reference's order and rounding,

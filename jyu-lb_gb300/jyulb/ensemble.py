@@ -3,9 +3,10 @@ relaxation time, body force and boundary set advanced together on one GPU.
 
 The reference advances one ``Solver`` at a time (jyulb/isothermal.pyx:
 1370-1418); an ensemble there is a Python loop over Solver objects.  Here all
-domains share one packed node index, one FP32-shifted population array and one
-kernel launch per time step (graph-replayed), with the block size chosen by a
-timing autotuner at set-up.
+domains share one packed node index and one FP32-shifted population array.  One
+kernel launch advances all of them a time step (graph-replayed), or, in longer
+calls on ensembles larger than the L2, a group of them that stays in it.  The
+block size is chosen by a timing autotuner at set-up.
 
 Each domain is described like a Solver: interior ``phase``, ``den`` and
 ``vel`` arrays (k fastest), ``kvisc``, gravity ``g`` and per-face ``bc``
